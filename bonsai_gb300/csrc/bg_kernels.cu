@@ -41,11 +41,11 @@ struct TraceSrc {
 };
 
 // LAYOUT: 1 = reference binary layout, 2 = 2-wide, 8 = 8-wide compressed.
-// Traversal kernels are capped at 64 registers (8 blocks of 128 threads per SM): occupancy hides
-// the node-fetch latency better than the extra registers would (measured on the production scene:
-// -20% frame time against the uncapped 96-register build).
+// Traversal kernels are compiled for 7 blocks of 128 threads per SM (72 registers): with 8 (64
+// registers) they spill, with 6 (80) too few warps hide the node fetches.  Ray microbenchmark
+// 12.84 ms against 14.37 with 8 and 14.05 with 6; production frame at 16 spp 106.7 / 109.1 / 110.7 ms.
 #ifndef BG_MINBLOCKS
-#define BG_MINBLOCKS 8
+#define BG_MINBLOCKS 7
 #endif
 template <int LAYOUT, bool ANY>
 __global__ void __launch_bounds__(128, BG_MINBLOCKS) k_trace(Scene sc, const float4* rays, uint32_t n, int2* hits, uint8_t* occ,

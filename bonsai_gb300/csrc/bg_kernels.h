@@ -139,7 +139,10 @@ struct LaunchShape {
     int sms;
     int block;
     int blocks_per_sm = 8;
-    int refill = 32;
+    // Traversal fetches new rays once this many lanes of a warp are idle.  8 against 32 (whole warps
+    // only): ray microbenchmark 13.8 against 19.0 ms, production frame 115.2 / 131.2 ms, guided slit
+    // room 11.9 / 12.9 ms; 4 and 16 lose 1-7% to 8; the Cornell box (16 primitives) loses 1%.
+    int refill = 8;
     int sort_rays = 0;
     int l2_persist = 0;  // BG_TUNE_L2_PERSIST (part of the captured graph's key)
     // BG_TUNE_TILE_PIXELS, on by default: production 1080p at 16 spp 169.4 ms against 174.1 ms in

@@ -18,7 +18,7 @@
 #include "bg_tree_wave.cuh"
 
 #ifndef BG_MINBLOCKS
-#define BG_MINBLOCKS 8
+#define BG_MINBLOCKS 7  // as bg_kernels.cu
 #endif
 
 namespace bg {
