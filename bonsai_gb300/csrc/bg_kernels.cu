@@ -361,14 +361,17 @@ __global__ void __launch_bounds__(256) k_sort_scatter(WaveBuffers wb, RenderPara
 // shade launch runs one material's code with uniform control flow.  GWK (guided waves, queries
 // set): a hit of a guidable class (matte, plastic, conductor) also writes its network query at
 // class * gw.cap + its queue position, for the inference that runs before shading.
+constexpr uint32_t BIN_BLOCK = 512;
 template <bool MULTI = false, bool GWK = false>
-__global__ void __launch_bounds__(128) k_bin(Scene sc0, WaveBuffers wb, uint32_t bounce, const SceneRender* tab,
-                                             GuideWave gw = GuideWave{}, bool queries = false) {
+__global__ void __launch_bounds__(BIN_BLOCK) k_bin(Scene sc0, WaveBuffers wb, uint32_t bounce, const SceneRender* tab,
+                                                   GuideWave gw = GuideWave{}, bool queries = false) {
     const uint32_t n = wb.counters[bounce & 1];
     const uint32_t* q = wb.queue[bounce & 1];
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += stride) {
-        uint32_t i = base + lane_id();
+    __shared__ BlockAppend<NCLS> append;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        __syncthreads();
+        const uint32_t i = base + threadIdx.x;
         int cls = -1;
         uint32_t slot = 0;
         if (i < n) {
@@ -377,13 +380,15 @@ __global__ void __launch_bounds__(128) k_bin(Scene sc0, WaveBuffers wb, uint32_t
             const Scene& sc = pick<MULTI>(sc0, MULTI ? &tab[wb.scene_id[slot]].sc : nullptr);
             cls = prim < 0 ? CLS_MISS : (int)sc.prim_cls[prim];
         }
-        uint32_t qpos = 0;
+        uint32_t qpos = 0, pos[NCLS];
+        append({&wb.counters[C_CLS], &wb.counters[C_CLS + 1], &wb.counters[C_CLS + 2], &wb.counters[C_CLS + 3],
+                &wb.counters[C_CLS + 4]},
+               {cls == 0, cls == 1, cls == 2, cls == 3, cls == 4}, pos);
 #pragma unroll
         for (int c = 0; c < NCLS; ++c) {
-            uint32_t pos = warp_append(&wb.counters[C_CLS + c], cls == c);
             if (cls == c) {
-                wb.cls_queue[(size_t)c * wb.capacity + pos] = slot;
-                qpos = (uint32_t)c * gw.cap + pos;
+                wb.cls_queue[(size_t)c * wb.capacity + pos[c]] = slot;
+                qpos = (uint32_t)c * gw.cap + pos[c];
             }
         }
         // one intersection per lane (outside the class loop, so the lanes of all three classes
@@ -470,6 +475,7 @@ static int launch_bounces(const Scene& sc, const RenderParams& rp, const FilmBuf
                           uint32_t* err, const LaunchShape& ls, cudaStream_t s, cudaEvent_t* ev, const GuideWave* gwp) {
     int launches = 0;
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
+    const dim3 bin_grid(ls.sms * 4);  // 2048 threads per SM
     const GuideWave gw = gwp ? *gwp : GuideWave{};
     const bool guided = (gw.flags & GW_GUIDED) != 0;
     for (uint32_t b = 0; b <= rp.max_depth; ++b) {
@@ -488,15 +494,15 @@ static int launch_bounces(const Scene& sc, const RenderParams& rp, const FilmBuf
         if (queries) {
             // every hit of a guidable class queues its network query; the network's mixtures are
             // ready before the shade launches
-            k_bin<false, true><<<grid, block, 0, s>>>(sc, wb, b, nullptr, gw, true);
+            k_bin<false, true><<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, nullptr, gw, true);
             launch_guide_infer(gw.wpack, gw.query, &wb.counters[C_CLS], 3, gw.cap, gw.raw, true, err, ls.sms, s);
             launches += 1;
         } else {
-            k_bin<<<grid, block, 0, s>>>(sc, wb, b, nullptr);
+            k_bin<<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, nullptr);
         }
         if (ev) cudaEventRecord(ev[4 * b + 1], s);
-        if (gw.flags) launches += launch_shade_guided(sc, rp, film, wb, gw, b, err, grid, block, s, ls.fork);
-        else launches += launch_shade_plain(sc, rp, film, wb, b, err, grid, block, s, ls.fork);
+        if (gw.flags) launches += launch_shade_guided(sc, rp, film, wb, gw, b, err, grid, s, ls.fork);
+        else launches += launch_shade_plain(sc, rp, film, wb, b, err, grid, s, ls.fork);
         if (ev) cudaEventRecord(ev[4 * b + 2], s);
         if (sc.nodes8) k_shadow<8><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
         else k_shadow<2><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
@@ -523,13 +529,14 @@ int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_dep
     const Scene sc{};
     const FilmBuffers film{};
     const GuideWave gw{};
+    const dim3 bin_grid(ls.sms * 4);
     k_generate_batch<<<grid, block, 0, s>>>(tab, nscenes, wb, item0, nitems);
     int launches = 1;
     for (uint32_t b = 0; b <= max_depth; ++b) {
         k_prepare<<<1, 32, 0, s>>>(wb, b);
         k_extend<8, true><<<grid, block, 0, s>>>(sc, wb, b, err, ls.refill, tab, false);
-        k_bin<true><<<grid, block, 0, s>>>(sc, wb, b, tab);
-        launch_shade_batch(tab, wb, b, err, grid, block, s, variants != 0);
+        k_bin<true><<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, tab);
+        launch_shade_batch(tab, wb, b, err, grid, s, variants != 0);
         k_shadow<8, true><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, tab);
         k_finalize<true><<<grid, block, 0, s>>>(sc, film, wb, gw, tab);
         launches += 10;

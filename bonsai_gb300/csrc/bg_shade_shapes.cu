@@ -6,13 +6,14 @@
 namespace bg {
 
 int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        uint32_t b, uint32_t* err, dim3 grid, dim3 block, cudaStream_t s) {
+                        uint32_t b, uint32_t* err, dim3 grid, cudaStream_t s) {
+    const dim3 sg = shade_grid(grid);
     const GuideWave gw{};
-    k_shade<CLS_MISS><<<grid, block, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<0, false, false, true, true, true><<<grid, block, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<1, false, false, true, true, true><<<grid, block, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<2, false, false, false, true, true><<<grid, block, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<3, false, false, false, true, true><<<grid, block, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
+    k_shade<CLS_MISS><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
+    k_shade<0, false, false, true, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
+    k_shade<1, false, false, true, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
+    k_shade<2, false, false, false, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
+    k_shade<3, false, false, false, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
     return 5;
 }
 

@@ -15,6 +15,8 @@
 // so both produce the same estimate for every sample up to float summation order.  The direct
 // strategy of MIS through the BSDF becomes an occlusion ray up to the light (the light's own
 // triangle skipped), as in the path wavefront.
+#include <algorithm>
+
 #include "bg_tree_wave.cuh"
 
 #ifndef BG_MINBLOCKS
@@ -134,13 +136,14 @@ int launch_tree_wave(int kind, const Scene& sc, const Camera& cam, const RenderP
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_tw_gen<<<grid, block, 0, s>>>(cam, rp, tw, item0, n);
     ++launches;
+    const dim3 shade_grid(std::max(1u, (uint32_t)(ls.sms * ls.blocks_per_sm) * 128u / TW_SHADE_BLOCK));
     const bool wide8 = sc.nodes8 != nullptr;
     for (uint32_t d = 0; d < rp.max_depth; ++d) {
         k_tw_prep<<<1, 1, 0, s>>>(tw, d);
         if (wide8) k_tw_extend<8><<<grid, block, 0, s>>>(sc, tw, d, err, ls.refill);
         else k_tw_extend<2><<<grid, block, 0, s>>>(sc, tw, d, err, ls.refill);
-        if (kind == 1) launch_tw_shade_whitted(sc, rp, tw, d, item0, err, grid, block, s);
-        else launch_tw_shade_direct(kind, sc, rp, tw, d, item0, err, grid, block, s);
+        if (kind == 1) launch_tw_shade_whitted(sc, rp, tw, d, item0, err, shade_grid, s);
+        else launch_tw_shade_direct(kind, sc, rp, tw, d, item0, err, shade_grid, s);
         if (wide8) k_tw_shadow<8><<<grid, block, 0, s>>>(sc, tw, err, ls.refill);
         else k_tw_shadow<2><<<grid, block, 0, s>>>(sc, tw, err, ls.refill);
         launches += 4;

@@ -36,41 +36,53 @@ BG_D void add_L(const TreeWave& tw, uint32_t slot, RGB c) {
     atomicAdd(&tw.L[slot].z, c.b);
 }
 
-// Appends a shadow ray (warp-collective: every lane calls it, lanes without a ray pass has = false).
-BG_D void push_shadow(const TreeWave& tw, bool has, const Ray& r, int skip, RGB c, uint32_t slot) {
-    const uint32_t pos = warp_append(&tw.counters[TW_SHADOW], has);
-    if (!has) return;
-    if (pos >= tw.sh_cap) {
-        atomicOr(&tw.counters[TW_OVERFLOW], 1u);
-        return;
+// Up to two shadow rays per thread, appended for the whole block (every thread calls it).
+struct TwShadow {
+    bool has = false;
+    Ray r;
+    int skip = -1;
+    RGB c;
+};
+BG_D void push_shadows(const TreeWave& tw, const TwShadow (&sh)[2], uint32_t slot, BlockAppend<2>& append) {
+    uint32_t pos[2];
+    append({&tw.counters[TW_SHADOW], &tw.counters[TW_SHADOW]}, {sh[0].has, sh[1].has}, pos);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (!sh[k].has) continue;
+        if (pos[k] >= tw.sh_cap) {
+            atomicOr(&tw.counters[TW_OVERFLOW], 1u);
+            continue;
+        }
+        const Ray& r = sh[k].r;
+        tw.sh_o[pos[k]] = make_float4(r.o.x, r.o.y, r.o.z, r.t_max);
+        tw.sh_d[pos[k]] = make_float4(r.d.x, r.d.y, r.d.z, __int_as_float(sh[k].skip));
+        tw.sh_c[pos[k]] = make_float4(sh[k].c.r, sh[k].c.g, sh[k].c.b, __uint_as_float(slot));
     }
-    tw.sh_o[pos] = make_float4(r.o.x, r.o.y, r.o.z, r.t_max);
-    tw.sh_d[pos] = make_float4(r.d.x, r.d.y, r.d.z, __int_as_float(skip));
-    tw.sh_c[pos] = make_float4(c.r, c.g, c.b, __uint_as_float(slot));
 }
 
 // estimate_direct (src/base/integrator.rs:330-437, PBRT) for one light as up to two shadow rays:
 // the light sample's visibility ray and the BSDF sample's occlusion ray up to the light.  Both
-// contributions are scaled by `scale` (beta / light-selection pdf).  Warp-collective.
+// contributions are scaled by `scale` (beta / light-selection pdf).  Block-collective.
 BG_D void direct_rays(const Scene& sc, const TreeWave& tw, bool valid, const Isect& it, const BSDF& bsdf,
-                      uint32_t light_prim, float us0, float us1, float ul0, float ul1, RGB scale, uint32_t slot) {
+                      uint32_t light_prim, float us0, float us1, float ul0, float ul1, RGB scale, uint32_t slot,
+                      BlockAppend<2>& append) {
     const uint8_t flags = BSDF_ALL & ~BSDF_SPECULAR;
-    bool h0 = false, h1 = false;
-    Ray r0, r1;
-    RGB c0 = rgb(0.0f), c1 = rgb(0.0f);
+    TwShadow sh[2];
     if (valid) {
         LightSample ls = light_sample_any<false>(sc, light_prim, it, ul0, ul1);
-        float scattering_pdf = 0.0f;
         if (ls.pdf > 0.0f && !is_black(ls.radiance)) {
             RGB f = bsdf.f<false>(it.wo, ls.wi, flags) * abs_dot(ls.wi, it.ns);
-            scattering_pdf = bsdf.pdf<false>(it.wo, ls.wi, flags);
+            const float scattering_pdf = bsdf.pdf<false>(it.wo, ls.wi, flags);
             if (!is_black(f)) {
                 float w = power_heuristic(1.0f, ls.pdf, 1.0f, scattering_pdf);
-                c0 = scale * (f * ls.radiance * w / ls.pdf);
-                r0 = spawn_ray_to(it.p, it.p_err, it.n, it.time, ls.pt.p, ls.pt.p_err, ls.pt.n);
-                h0 = true;
+                sh[0].c = scale * (f * ls.radiance * w / ls.pdf);
+                sh[0].r = spawn_ray_to(it.p, it.p_err, it.n, it.time, ls.pt.p, ls.pt.p_err, ls.pt.n);
+                sh[0].has = true;
             }
         }
+    }
+    __syncthreads();
+    if (valid) {
         BxSample bs = bsdf.sample<false>(it.wo, us0, us1, flags);
         RGB f = bs.f * abs_dot(bs.wi, it.ns);
         if (!is_black(f) && bs.pdf > 0.0f) {
@@ -81,39 +93,42 @@ BG_D void direct_rays(const Scene& sc, const TreeWave& tw, bool valid, const Ise
                 float w = power_heuristic(1.0f, bs.pdf, 1.0f, lpdf);
                 RGB li = light_radiance_along(sc, light_prim, bs.wi, ln);
                 if (!is_black(li)) {
-                    c1 = scale * (f * li * w / bs.pdf);
-                    r1 = spawn_ray(it.p, it.p_err, it.n, it.time, bs.wi, false);
-                    r1.t_max = t_light;
-                    h1 = true;
+                    sh[1].c = scale * (f * li * w / bs.pdf);
+                    sh[1].r = spawn_ray(it.p, it.p_err, it.n, it.time, bs.wi, false);
+                    sh[1].r.t_max = t_light;
+                    sh[1].skip = light_prim == LIGHT_INFINITE ? -1 : (int)light_prim;
+                    sh[1].has = true;
                 }
             }
         }
     }
-    push_shadow(tw, h0, r0, -1, c0, slot);
-    push_shadow(tw, h1, r1, light_prim == LIGHT_INFINITE ? -1 : (int)light_prim, c1, slot);
+    push_shadows(tw, sh, slot, append);
 }
 
 // Shades level d: emission, light sampling (kind 1 Whitted, 2 all lights, 3 one light) and the
 // specular children of level d + 1 (PBRT mode: the dielectric as SpecularReflection +
 // SpecularTransmission).
-// Compiled for 6 resident CTAs per SM (at most 80 registers): production 1080p, 64 spp, Whitted
-// 72.6 and direct lighting 36.8 Msamples/s, against 71.7 / 33.7 with 4 CTAs, 72.0 / 35.0 with 5
-// and 67.2 / 30.6 unconstrained (196 registers).
-#ifndef BG_TREE_SHADE_MINBLOCKS
-#define BG_TREE_SHADE_MINBLOCKS 6
-#endif
+// Bound by instruction fetch: the code is 540 KB and a warp reuses little of it, so all of an SM's
+// warps go through it together, one block of 1024 threads (64 registers, with spills) and a barrier
+// before each light, each light's second strategy and the children; a line fetched for one warp
+// serves 32.  Direct lighting on the production scene (640x360, 4 spp, depth 8): 21.2 ms with blocks
+// of 128 threads (6 per SM) that do not wait, 17.6 ms with barriers, 13.3 / 11.7 / 10.9 ms with blocks
+// of 384 / 768 / 1024, 10.3 ms with the barrier between the two strategies too.
+constexpr uint32_t TW_SHADE_BLOCK = 1024;
 // KIND: 1 Whitted, 2 direct lighting with UniformSampleAll, 3 with UniformSampleOne (each variant
 // carries only its own light-sampling code).
 template <bool TEX, int KIND>
-__global__ void __launch_bounds__(128, BG_TREE_SHADE_MINBLOCKS) k_tw_shade(Scene sc, RenderParams rp, TreeWave tw, uint32_t d,
+__global__ void __launch_bounds__(TW_SHADE_BLOCK, 1) k_tw_shade(Scene sc, RenderParams rp, TreeWave tw, uint32_t d,
                                                   uint64_t item0, uint32_t* err) {
     const uint32_t b = d & 1u, nb = b ^ 1u;
     const uint32_t n = min(tw.counters[b], tw.cap);
     const uint64_t npix = (uint64_t)rp.width * rp.height;
     const bool deeper = d + 1 < rp.max_depth;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += stride) {
-        const uint32_t i = base + lane_id();
+    __shared__ BlockAppend<2> append;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        __syncthreads();
+        const uint32_t i = base + threadIdx.x;
         bool valid = i < n;
         uint4 meta = make_uint4(0, 1, 0, 0);
         RGB beta = rgb(0.0f);
@@ -158,28 +173,29 @@ __global__ void __launch_bounds__(128, BG_TREE_SHADE_MINBLOCKS) k_tw_shade(Scene
         if (sc.nlights > 0) {
             if constexpr (KIND == 1) {  // whitted.rs:176-192
                 for (uint32_t j = 0; j < sc.nlights; ++j) {
-                    bool has = false;
-                    Ray sr;
-                    RGB c = rgb(0.0f);
+                    __syncthreads();
+                    TwShadow sh[2];
                     if (valid) {
                         LightSample ls = light_sample_any<false>(sc, sc.light_prims[j], it, rng.u(TW_DIM_LIGHTS + 2 * j),
                                                              rng.u(TW_DIM_LIGHTS + 2 * j + 1));
                         if (!is_black(ls.radiance) && ls.pdf != 0.0f) {
                             RGB f = bsdf.f<false>(it.wo, ls.wi, BSDF_ALL);
                             if (!is_black(f)) {
-                                c = beta * (f * ls.radiance * abs_dot(ls.wi, it.ns) / ls.pdf);
-                                sr = spawn_ray_to(it.p, it.p_err, it.n, it.time, ls.pt.p, ls.pt.p_err, ls.pt.n);
-                                has = true;
+                                sh[0].c = beta * (f * ls.radiance * abs_dot(ls.wi, it.ns) / ls.pdf);
+                                sh[0].r = spawn_ray_to(it.p, it.p_err, it.n, it.time, ls.pt.p, ls.pt.p_err, ls.pt.n);
+                                sh[0].has = true;
                             }
                         }
                     }
-                    push_shadow(tw, has, sr, -1, c, slot);
+                    push_shadows(tw, sh, slot, append);
                 }
             } else if constexpr (KIND == 2) {  // uniform_sample_all_lights (integrator.rs:274-307)
                 for (uint32_t j = 0; j < sc.nlights; ++j) {
+                    __syncthreads();
                     float u[4];
                     rng.block(TW_DIM_LIGHTS + 4 * j, u);
-                    direct_rays(sc, tw, valid, it, bsdf, sc.light_prims[j], u[2], u[3], u[0], u[1], beta / 1.0f, slot);
+                    direct_rays(sc, tw, valid, it, bsdf, sc.light_prims[j], u[2], u[3], u[0], u[1], beta / 1.0f, slot,
+                                append);
                 }
             } else {  // uniform_sample_one_light (integrator.rs:309-328)
                 float u[8];
@@ -188,42 +204,57 @@ __global__ void __launch_bounds__(128, BG_TREE_SHADE_MINBLOCKS) k_tw_shade(Scene
                 const float count = (float)sc.nlights;
                 const uint32_t li = (uint32_t)rmin(u[0] * count, count - 1.0f);
                 direct_rays(sc, tw, valid, it, bsdf, sc.light_prims[li], u[3], u[4], u[1], u[2], beta / (1.0f / count),
-                            slot);
+                            slot, append);
             }
         }
-        // specular children (specular_reflect / specular_transmit, integrator.rs:143-272)
-        for (int k = 0; k < 2; ++k) {
-            bool has = false;
-            BxSample bs;
-            if (valid && deeper) {
-                float us[4];
-                rng.block(TW_DIM_SPEC, us);
+        // specular children (specular_reflect / specular_transmit, integrator.rs:143-272), the same code
+        // for both (one copy in the instruction cache)
+        __syncthreads();
+        BxSample bs2[2];
+        bool has[2] = {false, false};
+        if (valid && deeper) {
+            float us[4];
+            rng.block(TW_DIM_SPEC, us);
+#pragma unroll 1
+            for (int k = 0; k < 2; ++k) {
                 const uint8_t type = k == 0 ? (BSDF_REFLECTION | BSDF_SPECULAR) : (BSDF_TRANSMISSION | BSDF_SPECULAR);
-                bs = bsdf.sample<false>(it.wo, us[2 * k], us[2 * k + 1], type);
-                has = bs.pdf > 0.0f && !is_black(bs.f) && abs_dot(bs.wi, it.ns) != 0.0f;
+                const BxSample bs = bsdf.sample<false>(it.wo, k ? us[2] : us[0], k ? us[3] : us[1], type);
+                const bool h = bs.pdf > 0.0f && !is_black(bs.f) && abs_dot(bs.wi, it.ns) != 0.0f;
+                if (k) {
+                    bs2[1] = bs;
+                    has[1] = h;
+                } else {
+                    bs2[0] = bs;
+                    has[0] = h;
+                }
             }
-            const uint32_t pos = warp_append(&tw.counters[nb], has);
-            if (!has) continue;
-            if (pos >= tw.cap) {
+        }
+        uint32_t pos[2];
+        append({&tw.counters[nb], &tw.counters[nb]}, has, pos);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!has[k]) continue;
+            if (pos[k] >= tw.cap) {
                 atomicOr(&tw.counters[TW_OVERFLOW], 1u);
                 continue;
             }
+            const BxSample& bs = bs2[k];
             const Ray c = spawn_ray(it.p, it.p_err, it.n, it.time, bs.wi, false);
             const RGB cb = beta * (bs.f * abs_dot(bs.wi, it.ns) / bs.pdf);
-            tw.ray_o[nb][pos] = make_float4(c.o.x, c.o.y, c.o.z, c.t_max);
-            tw.ray_d[nb][pos] = make_float4(c.d.x, c.d.y, c.d.z, c.time);
-            tw.beta[nb][pos] = make_float4(cb.r, cb.g, cb.b, 0.0f);
+            tw.ray_o[nb][pos[k]] = make_float4(c.o.x, c.o.y, c.o.z, c.t_max);
+            tw.ray_d[nb][pos[k]] = make_float4(c.d.x, c.d.y, c.d.z, c.time);
+            tw.beta[nb][pos[k]] = make_float4(cb.r, cb.g, cb.b, 0.0f);
             const bool crd = TEX && has_rd && have_tp;
-            tw.meta[nb][pos] = make_uint4(slot, 2u * node + (uint32_t)k, d + 1, crd ? 1u : 0u);
-            if (crd) store_rd(tw.rd[nb], pos, specular_diff(it, tp, rd, bs.wi, bsdf.eta, k == 1));
+            tw.meta[nb][pos[k]] = make_uint4(slot, 2u * node + (uint32_t)k, d + 1, crd ? 1u : 0u);
+            if (crd) store_rd(tw.rd[nb], pos[k], specular_diff(it, tp, rd, bs.wi, bsdf.eta, k == 1));
         }
     }
 }
 
 // Launches the shade kernel of level d for integrator `kind` (bg_tree_shade_w.cu, bg_tree_shade_d.cu).
 void launch_tw_shade_whitted(const Scene& sc, const RenderParams& rp, const TreeWave& tw, uint32_t d, uint64_t item0,
-                             uint32_t* err, dim3 grid, dim3 block, cudaStream_t s);
+                             uint32_t* err, dim3 grid, cudaStream_t s);
 void launch_tw_shade_direct(int kind, const Scene& sc, const RenderParams& rp, const TreeWave& tw, uint32_t d,
-                            uint64_t item0, uint32_t* err, dim3 grid, dim3 block, cudaStream_t s);
+                            uint64_t item0, uint32_t* err, dim3 grid, cudaStream_t s);
 
 }  // namespace bg

@@ -24,6 +24,46 @@ BG_D uint32_t warp_append(uint32_t* counter, bool pred) {
     return base + (uint32_t)__popc(mask & ((1u << lane_id()) - 1u));
 }
 
+// Appends of a whole block to NQ queues with one atomic per queue: thread t enters counters[c]'s queue
+// when pred[c], at pos[c].  Every thread of the block calls it (two barriers); `sm` is the block's
+// scratch, free again after the next barrier.  Queue counters are single addresses, and a counter
+// takes about one atomic per nanosecond from the whole GPU: one per warp and queue bound the binning
+// and most of the shading (2^20 Cornell box paths: binning 38 us a bounce, 3 us of memory traffic).
+template <int NQ>
+struct BlockAppend {
+    uint32_t n[NQ][32];  // per queue and warp: lanes that append, then the warp's first position
+    BG_D void operator()(uint32_t* const (&counters)[NQ], const bool (&pred)[NQ], uint32_t (&pos)[NQ]) {
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31u) >> 5;
+        uint32_t mask[NQ];
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) {
+            mask[c] = __ballot_sync(FULL, pred[c]);
+            if (lane == 0) n[c][warp] = __popc(mask[c]);
+        }
+        __syncthreads();
+        for (uint32_t c = warp; c < (uint32_t)NQ; c += nwarps) {  // a warp scans a queue's counts
+            const uint32_t own = lane < nwarps ? n[c][lane] : 0u;
+            uint32_t incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= (uint32_t)o) incl += t;
+            }
+            uint32_t base = 0;
+            if (lane == 31 && incl) {
+#pragma unroll
+                for (int k = 0; k < NQ; ++k)
+                    if (c == (uint32_t)k) base = atomicAdd(counters[k], incl);
+            }
+            base = __shfl_sync(FULL, base, 31);
+            if (lane < nwarps) n[c][lane] = base + incl - own;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) pos[c] = n[c][warp] + __popc(mask[c] & ((1u << lane) - 1u));
+    }
+};
+
 BG_D Ray load_ray(float4 o, float4 d) {
     Ray r;
     r.o = f4xyz(o);

@@ -15,6 +15,16 @@
 
 namespace bg {
 
+// Threads per block of the shade kernels, whose warps go through the code side by side (a barrier at
+// every path): their code is 100 to 550 KB, far beyond the instruction caches, and a line fetched
+// for one warp serves the others of the block only while they are near it.  One block of 512 per SM
+// against four of 128: textured room 3.43 / 3.99 ms, guided slit room 9.34 / 10.04 ms, production
+// frame at 16 spp 94.6 / 96.0 ms (256: 3.63, 9.65, 95.0); the example scene, whose paths mostly
+// escape at once, loses 2%.  More barriers, between the parts of a vertex, cost more than they give.
+constexpr uint32_t SHADE_BLOCK = 512;
+// Grid of SHADE_BLOCK-thread blocks with the threads of `grid` blocks of 128.
+inline dim3 shade_grid(dim3 grid) { return dim3(grid.x * 128u / SHADE_BLOCK > 0 ? grid.x * 128u / SHADE_BLOCK : 1u); }
+
 // ================================================================ textures
 // Texture inputs at a hit whose material is textured (nullptr otherwise): the surface geometry
 // re-derived from the hit and the screen-space differentials of ray differentials `rd`.
@@ -273,7 +283,7 @@ struct VertexOut {
 // 1D k1 + 1; without, the BSDF's 2D k2 and the roulette's 1D k1), -1 where the call falls through to
 // the counter RNG.  A shade thread computes them when it picks up a path, where few registers are
 // live, into its column of shared memory (8 rows, stride SU_STRIDE).
-constexpr uint32_t SU_STRIDE = 128;
+constexpr uint32_t SU_STRIDE = SHADE_BLOCK;
 // Not inlined: renders with the independent sampler never call it, and its code (permutations, cycle
 // walking) would otherwise sit among the shade kernels' hot instructions.
 static __device__ __noinline__ void strat_prefetch(const StratParams& sp, uint32_t pix, uint32_t sample, uint64_t seed, uint32_t k1,
@@ -470,22 +480,23 @@ BG_D void scatter_vertex(const Scene& sc, const RenderParams& rp, const WaveBuff
     out.cont = true;
 }
 
-// Warp-convergent tail of k_shade: queue compaction, shadow rays, records.
+// Block-convergent tail of k_shade: queue compaction, shadow rays, records.
 // lrec: this lane's path resolved a visible light-sample record of its previous vertex.
 BG_D void finish_vertex(const WaveBuffers& wb, const GuideWave& gw, uint32_t bounce, uint32_t slot, bool cont,
                         bool done_pending, const VertexOut& vo, uint32_t emit_n, RGB L_emit, bool record,
-                        uint32_t* err, bool lrec = false) {
-    uint32_t pos = warp_append(&wb.counters[(bounce + 1) & 1], cont);
-    if (cont) wb.queue[(bounce + 1) & 1][pos] = slot;
-    pos = warp_append(&wb.counters[C_DONE], done_pending);
-    if (done_pending) wb.done[pos] = slot;
+                        uint32_t* err, bool lrec, BlockAppend<4>& append) {
+    uint32_t pos[4];
+    append({&wb.counters[(bounce + 1) & 1], &wb.counters[C_DONE], &wb.counters[C_SHADOW], &wb.counters[C_SHADOW]},
+           {cont, done_pending, vo.push_sh[0], vo.push_sh[1]}, pos);
+    if (cont) wb.queue[(bounce + 1) & 1][pos[0]] = slot;
+    if (done_pending) wb.done[pos[1]] = slot;
+#pragma unroll
     for (int k = 0; k < 2; ++k) {
-        pos = warp_append(&wb.counters[C_SHADOW], vo.push_sh[k]);
         if (vo.push_sh[k]) {
-            if (pos < wb.sh_capacity) {
-                wb.sh_o[pos] = vo.sh_o[k];
-                wb.sh_d[pos] = vo.sh_d[k];
-                wb.sh_ref[pos] = 2 * slot + (uint32_t)k;
+            if (pos[2 + k] < wb.sh_capacity) {
+                wb.sh_o[pos[2 + k]] = vo.sh_o[k];
+                wb.sh_d[pos[2 + k]] = vo.sh_d[k];
+                wb.sh_ref[pos[2 + k]] = 2 * slot + (uint32_t)k;
             } else {
                 atomicOr(err, ERR_QUEUE_OVERFLOW);
             }
@@ -513,7 +524,7 @@ BG_D void finish_vertex(const WaveBuffers& wb, const GuideWave& gw, uint32_t bou
 #define BG_GUIDED_SHADE_MINBLOCKS 4
 #endif
 template <int CLS, bool MULTI = false, bool GWK = false, bool TEX = false, bool INF = false, bool SHL = INF>
-__global__ void __launch_bounds__(128, GWK ? BG_GUIDED_SHADE_MINBLOCKS : BG_SHADE_MINBLOCKS) k_shade(Scene sc0, RenderParams rp0, FilmBuffers film0, WaveBuffers wb,
+__global__ void __launch_bounds__(SHADE_BLOCK, (GWK ? BG_GUIDED_SHADE_MINBLOCKS : BG_SHADE_MINBLOCKS) * 128 / SHADE_BLOCK) k_shade(Scene sc0, RenderParams rp0, FilmBuffers film0, WaveBuffers wb,
                                                GuideWave gw, uint32_t bounce, uint32_t* err, const SceneRender* tab) {
     constexpr bool GUIDABLE = CLS >= 0 && CLS <= 2;
     const uint32_t n = wb.counters[C_CLS + CLS];
@@ -522,9 +533,11 @@ __global__ void __launch_bounds__(128, GWK ? BG_GUIDED_SHADE_MINBLOCKS : BG_SHAD
     __shared__ float strat_su[CLS != CLS_MISS ? 8 * SU_STRIDE : 1];
     const bool record = GWK && (gw.flags & GW_RECORD) != 0;
     const bool guided = GWK && GUIDABLE && (gw.flags & GW_GUIDED);
-    // warp-uniform loop so the ballots below see all 32 lanes
-    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += stride) {
-        uint32_t i = base + lane_id();
+    __shared__ BlockAppend<4> append;
+    // block-uniform loop: the barriers below see every thread
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        __syncthreads();
+        uint32_t i = base + threadIdx.x;
         bool active = i < n;
         uint32_t slot = active ? q[i] : 0;
         bool cont = false, done_pending = false, lrec_emit = false;
@@ -595,7 +608,7 @@ __global__ void __launch_bounds__(128, GWK ? BG_GUIDED_SHADE_MINBLOCKS : BG_SHAD
                 }
             }
         }
-        finish_vertex(wb, gw, bounce, slot, cont, done_pending, vo, emit_n, L_emit, record, err, lrec_emit);
+        finish_vertex(wb, gw, bounce, slot, cont, done_pending, vo, emit_n, L_emit, record, err, lrec_emit, append);
     }
 }
 
@@ -629,21 +642,19 @@ inline void shade_join(cudaStream_t s, const ShadeFork* fork) {
 
 // Single-scene shade launches for scenes with emitting spheres or quadrics (bg_shade_shapes.cu).
 int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        uint32_t bounce, uint32_t* err, dim3 grid, dim3 block, cudaStream_t s);
+                        uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s);
 // Shade launches of one bounce (the five material classes, misses included); with `fork` the
 // classes run on parallel streams, joined back into `s` before returning.
 int launch_shade_plain(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                       uint32_t bounce, uint32_t* err, dim3 grid, dim3 block, cudaStream_t s,
+                       uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s,
                        const ShadeFork* fork = nullptr);
 int launch_shade_guided(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, dim3 block, cudaStream_t s,
+                        const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s,
                         const ShadeFork* fork = nullptr);
 // The guided launches of scenes with textures or an infinite light (bg_shade_guided_full.cu).
 int launch_shade_guided_full(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                             const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, dim3 block,
-                             cudaStream_t s, const ShadeFork* fork = nullptr);
+                             const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s, const ShadeFork* fork = nullptr);
 // full: the variants that handle textured scenes and infinite lights (checked per path's scene).
-int launch_shade_batch(const SceneRender* tab, const WaveBuffers& wb, uint32_t bounce, uint32_t* err, dim3 grid,
-                       dim3 block, cudaStream_t s, bool full);
+int launch_shade_batch(const SceneRender* tab, const WaveBuffers& wb, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s, bool full);
 
 }  // namespace bg
