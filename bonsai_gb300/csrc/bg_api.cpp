@@ -287,7 +287,6 @@ bg_status ensure_wave(bg_ctx* ctx, uint32_t cap) {
     WB(queue[0], n * sizeof(uint32_t));
     WB(queue[1], n * sizeof(uint32_t));
     WB(cls_queue, 5 * n * sizeof(uint32_t));
-    WB(done, n * sizeof(uint32_t));
     WB(counters, 16 * sizeof(uint32_t));
     WB(ray_stats, 4 * sizeof(unsigned long long));
     WB(wavectl, 4 * sizeof(uint32_t));
@@ -1195,6 +1194,7 @@ bg_status bg_scene_commit(bg_scene* s, uint32_t kind, bg_build_stats* stats) {
         for (uint32_t i = 0; i < ntri; ++i) cls[i] = (uint8_t)mats[s->tri_mat[i]].type;
         for (uint32_t i = 0; i < nsph; ++i) cls[ntri + i] = (uint8_t)mats[sph_mat[i]].type;
         for (uint32_t i = 0; i < nquad; ++i) cls[ntri + nsph + i] = (uint8_t)mats[s->quads[i].material_id].type;
+        for (uint8_t c : cls) d.cls_mask |= 1u << c;
         if (!cls.empty() && (st = upload(ctx, cls, &d.prim_cls, &s->allocs)) != BG_OK) return st;
     }
     if (any_sph_light && (st = upload(ctx, sph_emis, &d.sph_emis, &s->allocs)) != BG_OK) return st;
@@ -1590,7 +1590,7 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
     if (n > 65536) return fail(ctx, BG_ERR_INVALID, "at most 65536 scenes per batch");
     uint64_t total_pix = 0, total_items = 0;
     uint32_t max_depth = 0;
-    uint32_t variants = 0;  // bit 0: some scene is textured, bit 1: some scene holds an infinite light
+    uint32_t variants = 0;  // bit 0: some scene is textured, bit 1: some scene holds an infinite light, 2-5: material classes
     for (size_t i = 0; i < n; ++i) {
         const bg_batch_item& it = items[i];
         bg_render_opts o = it.opts;
@@ -1602,6 +1602,7 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
         if (it.opts.mode != BG_MODE_PBRT) return fail(ctx, BG_ERR_UNSUPPORTED, "batch rendering needs BG_MODE_PBRT");
         if (it.opts.integrator != BG_INTEGRATOR_PATH)
             return fail(ctx, BG_ERR_UNSUPPORTED, "batch rendering runs the path integrator only");
+        variants |= it.scene->dev.cls_mask << 2;
         if (it.scene->dev.ntex) variants |= 1u;
         if (it.scene->has_inf || it.scene->dev.sph_emis || it.scene->dev.quad_emis) variants |= 2u;
         total_pix += (uint64_t)it.camera.width * it.camera.height;

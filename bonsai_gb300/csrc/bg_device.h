@@ -180,6 +180,7 @@ struct Scene {
     const float4* texels;
     const InfLight* inf;  // the infinite light, or null
     const uint8_t* prim_cls;  // material class (bg_material_type) per primitive: 1 B, stays in L2
+    uint32_t cls_mask;         // bit c: some primitive's material is of class c (bg_material_type)
 };
 
 enum : uint32_t {

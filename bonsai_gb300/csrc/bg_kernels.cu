@@ -1,7 +1,7 @@
 // bg_kernels.cu - ray-query kernels, the per-path megakernel and the PBRT wavefront stages.
 //
 // Wavefront (PBRT mode, 2-wide BVH):  one wave = up to `capacity` (pixel, sample) paths.
-//   generate -> [prepare -> extend -> shade -> shadow -> finalize] x (max_depth + 1)
+//   generate -> [extend -> bin -> shade -> shadow] x (max_depth + 1) -> film
 // Queue sizes live in device memory; every stage launches a fixed persistent grid that reads its
 // own work count, so the chain needs no host synchronisation and can be captured in a CUDA graph.
 // Traversal stages pull 32-ray batches per warp from an atomic head (dynamic load balance);
@@ -191,7 +191,10 @@ void launch_megakernel(bool ref_compat, const Scene& sc, const Camera& cam, cons
 // Batch: item -> scene by binary search over the scenes' first items, then as above.
 __global__ void k_generate_batch(const SceneRender* tab, uint32_t nscenes, WaveBuffers wb, uint64_t item0,
                                  uint32_t nitems) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) wb.counters[C_Q0] = nitems;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        wb.counters[C_Q0] = nitems;
+        wb.counters[C_EXT_HEAD] = 0;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
         const uint64_t item = item0 + i;
         uint32_t lo = 0, hi = nscenes - 1;
@@ -213,26 +216,22 @@ __global__ void k_generate(Camera cam, RenderParams rp, WaveBuffers wb, uint64_t
     generate_paths(cam, rp, wb, item0, nitems, rp.first_sample);
 }
 
-// Graph replay: the wave to generate comes from wb.wavectl (advanced by k_wave_advance).
-__global__ void k_generate_ctl(Camera cam, RenderParams rp, WaveBuffers wb, uint64_t total) {
+// Graph replay: the wave comes from wb.wavectl (advanced by k_wave_advance).
+struct WaveItems {
+    uint64_t item0;
+    uint32_t n;
+};
+BG_D WaveItems wave_items(const WaveBuffers& wb, uint64_t total) {
     const uint64_t item0 = (uint64_t)wb.wavectl[0] * wb.capacity;
-    const uint32_t nitems = item0 >= total ? 0u : (uint32_t)min((uint64_t)wb.capacity, total - item0);
-    generate_paths(cam, rp, wb, item0, nitems, wb.wavectl[1]);
+    return {item0, item0 >= total ? 0u : (uint32_t)min((uint64_t)wb.capacity, total - item0)};
+}
+__global__ void k_generate_ctl(Camera cam, RenderParams rp, WaveBuffers wb, uint64_t total) {
+    const WaveItems w = wave_items(wb, total);
+    generate_paths(cam, rp, wb, w.item0, w.n, wb.wavectl[1]);
 }
 
 __global__ void k_wave_advance(WaveBuffers wb) {
     if (threadIdx.x == 0) wb.wavectl[0] += 1;
-}
-
-__global__ void k_prepare(WaveBuffers wb, uint32_t bounce) {
-    if (threadIdx.x == 0) {
-        wb.counters[(bounce + 1) & 1] = 0;
-        wb.counters[C_SHADOW] = 0;
-        wb.counters[C_DONE] = 0;
-        wb.counters[C_EXT_HEAD] = 0;
-        wb.counters[C_SH_HEAD] = 0;
-        for (int c = 0; c < NCLS; ++c) wb.counters[C_CLS + c] = 0;
-    }
 }
 
 struct ExtendSrc {
@@ -252,7 +251,13 @@ template <int LAYOUT, bool MULTI = false>
 __global__ void __launch_bounds__(128, BG_MINBLOCKS) k_extend(Scene sc, WaveBuffers wb, uint32_t bounce, uint32_t* err,
                                                 int refill, const SceneRender* tab, bool sorted) {
     const uint32_t n = wb.counters[bounce & 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wb.ray_stats[0], (unsigned long long)n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(&wb.ray_stats[0], (unsigned long long)n);
+        wb.counters[(bounce + 1) & 1] = 0;
+        wb.counters[C_SHADOW] = 0;
+        wb.counters[C_SH_HEAD] = 0;
+        for (int c = 0; c < NCLS; ++c) wb.counters[C_CLS + c] = 0;
+    }
     ExtendSrc src{sorted ? wb.qsort : wb.queue[bounce & 1], wb, tab};
 #if BG_SMEM_STACK
     __shared__ uint2 stack8[LAYOUT == 8 ? STACK8 * 128 : 1];
@@ -369,6 +374,7 @@ __global__ void __launch_bounds__(BIN_BLOCK) k_bin(Scene sc0, WaveBuffers wb, ui
     const uint32_t* q = wb.queue[bounce & 1];
     const uint32_t stride = gridDim.x * blockDim.x;
     __shared__ BlockAppend<NCLS> append;
+    if (blockIdx.x == 0 && threadIdx.x == 0) wb.counters[C_EXT_HEAD] = 0;  // for the next bounce
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         __syncthreads();
         const uint32_t i = base + threadIdx.x;
@@ -441,45 +447,104 @@ __global__ void __launch_bounds__(128, BG_MINBLOCKS) k_shadow(Scene sc, WaveBuff
     else traverse_queue<true>(sc, n, &wb.counters[C_SH_HEAD], src, err, refill);
 }
 
-template <bool MULTI = false, bool GWK = false>
-__global__ void __launch_bounds__(128) k_finalize(Scene sc0, FilmBuffers film0, WaveBuffers wb, GuideWave gw,
-                                                  const SceneRender* tab, uint32_t bounce = 0) {
-    const uint32_t n = wb.counters[C_DONE];
-    const bool record = GWK && (gw.flags & GW_RECORD) != 0;
+// Recording waves, once all paths have ended: the records of the paths whose last vertex left a
+// light contribution pending (the others' were emitted when they ended) become training samples.
+__global__ void __launch_bounds__(128) k_emit_pending(Scene sc, WaveBuffers wb, GuideWave gw, uint32_t n) {
     for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += gridDim.x * blockDim.x) {
-        uint32_t i = base + lane_id();
-        uint32_t slot = 0, nrec = 0;
+        const uint32_t slot = base + lane_id();
+        uint32_t nrec = 0, bounce = 0;
         bool lrec = false;
         RGB L = rgb(0.0f);
-        if (i < n) {
-            slot = wb.done[i];
-            const SceneRender* sr = MULTI ? tab + wb.scene_id[slot] : nullptr;
-            const Scene& sc = pick<MULTI>(sc0, MULTI ? &sr->sc : nullptr);
-            const FilmBuffers& film = pick<MULTI>(film0, MULTI ? &sr->film : nullptr);
-            float4 l4 = wb.L[slot];
-            uint32_t state = wb.state[slot];
-            L = apply_pending(wb, slot, rgb(l4.x, l4.y, l4.z), state, sc.nlights);
-            film_add(film, wb.pixel[slot], L);
-            nrec = rec_count(state);
-            // the last vertex's light-sample record, resolved by this bounce's shadow rays
-            lrec = record && (state & ST_LREC) && wb.pending[2 * slot].w != 0.0f;
+        if (slot < n) {
+            const uint32_t state = wb.state[slot];
+            if (state & ST_PENDING) {
+                const float4 l4 = wb.L[slot];
+                L = apply_pending(wb, slot, rgb(l4.x, l4.y, l4.z), state, sc.nlights);
+                nrec = rec_count(state);
+                bounce = state & 0xFFu;
+                lrec = (state & ST_LREC) && wb.pending[2 * slot].w != 0.0f;
+            }
         }
-        if (record) {
-            emit_records(gw, wb, slot, nrec, L);
-            emit_light_record(gw, bounce, slot, lrec);
-        }
+        emit_records(gw, wb, slot, nrec, L);
+        emit_light_record(gw, bounce, slot, lrec);
     }
 }
 
-static int launch_bounces(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                          uint32_t* err, const LaunchShape& ls, cudaStream_t s, cudaEvent_t* ev, const GuideWave* gwp) {
+// Adds a wave's paths (items item0 .. item0 + n - 1 in slots 0 .. n - 1) to the film: their radiance
+// in L plus the last vertex's light contribution where its shadow rays have just resolved it, after
+// the radiance sanity checks of SamplerIntegrator::render (src/base/integrator.rs:91-120;
+// FilmTile::add_sample with the box filter, weight 1 to the sample's own pixel).  One thread adds all
+// of the wave's samples of a pixel, in sample order and without atomics (six FP64 atomics and one
+// integer one per path before: the Cornell box's contended 2^20 samples 0.12 ms of 1.86).
+// CTL: the wave is wb.wavectl's of `total` items.  MULTI: pixels and films of the path's scene.
+template <bool MULTI, bool CTL>
+__global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmBuffers film0, WaveBuffers wb,
+                                              uint64_t item0, uint32_t n, uint64_t total, const SceneRender* tab) {
+    if (CTL) {
+        const WaveItems w = wave_items(wb, total);
+        item0 = w.item0;
+        n = w.n;
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const SceneRender* sr = MULTI ? tab + wb.scene_id[i] : nullptr;
+        const RenderParams& rp = pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr);
+        const uint64_t npix = (uint64_t)rp.width * rp.height;
+        uint64_t first = 0, end = n;  // the scene's slots in this wave
+        if (MULTI) {
+            const uint64_t s0 = sr->item0, s1 = s0 + npix * rp.spp;
+            first = s0 > item0 ? s0 - item0 : 0;
+            end = min((uint64_t)n, s1 - item0);
+        }
+        if (i - first >= npix) {  // a later sample of its pixel
+            if (MULTI) continue;
+            break;
+        }
+        const uint32_t nlights = pick<MULTI>(sc0, MULTI ? &sr->sc : nullptr).nlights;
+        const FilmBuffers& f = pick<MULTI>(film0, MULTI ? &sr->film : nullptr);
+        double s[3] = {0.0, 0.0, 0.0}, q[3] = {0.0, 0.0, 0.0};
+        float ps[3] = {0.0f, 0.0f, 0.0f};
+        uint32_t cnt = 0, nan = 0;
+        for (uint64_t j = i; j < end; j += npix) {
+            const float4 l4 = wb.L[j];
+            RGB L = apply_pending(wb, (uint32_t)j, rgb(l4.x, l4.y, l4.z), wb.state[j], nlights);
+            const float y = luminance(L);
+            if (is_nan(L) || y < -1e-5f || isinf(y)) {
+                L = rgb(0.0f);
+                ++nan;
+            }
+            const double r = L.r, g = L.g, b = L.b;
+            s[0] += r;
+            s[1] += g;
+            s[2] += b;
+            q[0] += r * r;
+            q[1] += g * g;
+            q[2] += b * b;
+            ps[0] += L.r;
+            ps[1] += L.g;
+            ps[2] += L.b;
+            ++cnt;
+        }
+        const size_t pix = wb.pixel[i];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            f.sum[3 * pix + c] += s[c];
+            f.sumsq[3 * pix + c] += q[c];
+            if (f.pass) f.pass[3 * pix + c] += ps[c];
+        }
+        f.count[pix] += cnt;
+        if (nan) atomicAdd(f.nan_count, (unsigned long long)nan);
+    }
+}
+
+static int launch_bounces(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t* err,
+                          const LaunchShape& ls, cudaStream_t s, cudaEvent_t* ev, const GuideWave* gwp) {
     int launches = 0;
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     const dim3 bin_grid(ls.sms * 4);  // 2048 threads per SM
+    const uint32_t shade_blocks = 2 * (uint32_t)ls.sms;
     const GuideWave gw = gwp ? *gwp : GuideWave{};
     const bool guided = (gw.flags & GW_GUIDED) != 0;
     for (uint32_t b = 0; b <= rp.max_depth; ++b) {
-        k_prepare<<<1, 32, 0, s>>>(wb, b);
         if (ev) cudaEventRecord(ev[4 * b + 0], s);
         const bool sorted = ls.sort_rays && b > 0 && wb.qsort;
         if (sorted) {
@@ -501,15 +566,16 @@ static int launch_bounces(const Scene& sc, const RenderParams& rp, const FilmBuf
             k_bin<<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, nullptr);
         }
         if (ev) cudaEventRecord(ev[4 * b + 1], s);
-        if (gw.flags) launches += launch_shade_guided(sc, rp, film, wb, gw, b, err, grid, s, ls.fork);
-        else launches += launch_shade_plain(sc, rp, film, wb, b, err, grid, s, ls.fork);
+        if (gw.flags) launches += launch_shade_guided(sc, rp, wb, gw, b, err, shade_blocks, ls.fork, s);
+        else launches += launch_shade_plain(sc, rp, wb, b, err, shade_blocks, ls.fork, s);
         if (ev) cudaEventRecord(ev[4 * b + 2], s);
-        if (sc.nodes8) k_shadow<8><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
-        else k_shadow<2><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
+        if (b < rp.max_depth) {  // the last hits sample no light
+            if (sc.nodes8) k_shadow<8><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
+            else k_shadow<2><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, nullptr);
+            launches += 1;
+        }
         if (ev) cudaEventRecord(ev[4 * b + 3], s);
-        if (gw.flags) k_finalize<false, true><<<grid, block, 0, s>>>(sc, film, wb, gw, nullptr, b);
-        else k_finalize<<<grid, block, 0, s>>>(sc, film, wb, gw, nullptr);
-        launches += 5;
+        launches += 2;
     }
     return launches;
 }
@@ -519,7 +585,13 @@ int launch_wave(const Scene& sc, const Camera& cam, const RenderParams& rp, cons
                 cudaStream_t s, cudaEvent_t* ev, const GuideWave* gw) {
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_generate<<<grid, block, 0, s>>>(cam, rp, wb, item0, nitems);
-    return 1 + launch_bounces(sc, rp, film, wb, err, ls, s, ev, gw);
+    int launches = 2 + launch_bounces(sc, rp, wb, err, ls, s, ev, gw);
+    if (gw && (gw->flags & GW_RECORD)) {
+        k_emit_pending<<<grid, block, 0, s>>>(sc, wb, *gw, nitems);
+        launches += 1;
+    }
+    k_film<false, false><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, item0, nitems, 0, nullptr);
+    return launches;
 }
 
 int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_depth, const WaveBuffers& wb,
@@ -527,20 +599,21 @@ int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_dep
                       uint32_t variants) {
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     const Scene sc{};
+    const RenderParams rp{};
     const FilmBuffers film{};
-    const GuideWave gw{};
     const dim3 bin_grid(ls.sms * 4);
     k_generate_batch<<<grid, block, 0, s>>>(tab, nscenes, wb, item0, nitems);
-    int launches = 1;
+    int launches = 2;
     for (uint32_t b = 0; b <= max_depth; ++b) {
-        k_prepare<<<1, 32, 0, s>>>(wb, b);
         k_extend<8, true><<<grid, block, 0, s>>>(sc, wb, b, err, ls.refill, tab, false);
         k_bin<true><<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, tab);
-        launch_shade_batch(tab, wb, b, err, grid, s, variants != 0);
-        k_shadow<8, true><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, tab);
-        k_finalize<true><<<grid, block, 0, s>>>(sc, film, wb, gw, tab);
-        launches += 10;
+        launches += 2 + launch_shade_batch(tab, wb, b, err, variants >> 2, 2 * (uint32_t)ls.sms, ls.fork, s, (variants & 3u) != 0);
+        if (b < max_depth) {
+            k_shadow<8, true><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, tab);
+            launches += 1;
+        }
     }
+    k_film<true, false><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, item0, nitems, 0, tab);
     return launches;
 }
 
@@ -548,9 +621,10 @@ int launch_wave_chain(const Scene& sc, const Camera& cam, const RenderParams& rp
                       const WaveBuffers& wb, uint64_t total, uint32_t* err, const LaunchShape& ls, cudaStream_t s) {
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_generate_ctl<<<grid, block, 0, s>>>(cam, rp, wb, total);
-    int n = 1 + launch_bounces(sc, rp, film, wb, err, ls, s, nullptr, nullptr);
+    int n = 3 + launch_bounces(sc, rp, wb, err, ls, s, nullptr, nullptr);
+    k_film<false, true><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, 0, 0, total, nullptr);
     k_wave_advance<<<1, 32, 0, s>>>(wb);
-    return n + 1;
+    return n;
 }
 
 // ================================================================ film

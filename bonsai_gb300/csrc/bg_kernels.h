@@ -71,9 +71,8 @@ struct WaveBuffers {
     uint32_t* queue[2];
     uint32_t* cls_queue;  // 5 * capacity: hits binned by material class (matte, plastic, conductor,
                           // dielectric) and misses, written by extend, read by the class's shade launch
-    uint32_t* done;
-    uint32_t* counters; // [0,1] queue sizes, [2] shadow count, [3] done count, [4] extend head,
-                        // [5] shadow head, [6..10] class queue sizes, [11] guided queries
+    uint32_t* counters; // [0,1] queue sizes, [2] shadow count, [4] extend head, [5] shadow head,
+                        // [6..10] class queue sizes
     unsigned long long* ray_stats;  // [0] closest-hit rays traced, [1] any-hit rays traced
     uint32_t* wavectl;              // graph replay: [0] wave index, [1] first sample (device side)
     uint32_t* scene_id;             // batch renders: scene of each path slot
@@ -199,7 +198,7 @@ void launch_megakernel(bool ref_compat, const Scene& sc, const Camera& cam, cons
                        const FilmBuffers& film, uint32_t* err, const LaunchShape& ls, cudaStream_t s);
 // One wave of the PBRT wavefront: items [item0, item0 + nitems) of the pixel x sample space.
 // Returns the number of kernels launched.  stage_events (optional): 4 events per bounce, recorded
-// before extend, before shade, before shadow and before finalize.
+// before extend, before shade, before shadow and after it.
 // gw (optional): guiding state; guided waves write the network queries while binning and run the
 // network inference before the material shades of every bounce.
 int launch_wave(const Scene& sc, const Camera& cam, const RenderParams& rp, const FilmBuffers& film,
@@ -214,7 +213,7 @@ int launch_wave_chain(const Scene& sc, const Camera& cam, const RenderParams& rp
 // `nscenes` scenes (tab, device); paths of all scenes share the queues of one set of launches
 // (8-wide BVH layouts).  max_depth = the largest of the scenes'.  Returns the kernels launched.
 // variants: bit 0 some scene is textured, bit 1 some scene holds an infinite light (the shade
-// launches then take the variants that handle both per scene).
+// launches then take the variants that handle both per scene), bits 2-5 the scenes' material classes.
 int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_depth, const WaveBuffers& wb,
                       uint64_t item0, uint32_t nitems, uint32_t* err, const LaunchShape& ls, cudaStream_t s,
                       uint32_t variants = 0);

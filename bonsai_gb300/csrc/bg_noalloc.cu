@@ -64,8 +64,8 @@ constexpr size_t OFF_SH_REF = OFF_SH_D + align_up(2 * N * sizeof(float4));
 constexpr size_t OFF_Q0 = OFF_SH_REF + align_up(2 * N * sizeof(uint32_t));
 constexpr size_t OFF_Q1 = OFF_Q0 + align_up(N * sizeof(uint32_t));
 constexpr size_t OFF_CLS = OFF_Q1 + align_up(N * sizeof(uint32_t));
-constexpr size_t OFF_DONE = OFF_CLS + align_up(5 * N * sizeof(uint32_t));
-constexpr size_t SCRATCH_BYTES = OFF_DONE + align_up(N * sizeof(uint32_t));
+constexpr size_t OFF_SPARE = OFF_CLS + align_up(5 * N * sizeof(uint32_t));
+constexpr size_t SCRATCH_BYTES = OFF_SPARE + align_up(N * sizeof(uint32_t));  // the published size
 static_assert(SCRATCH_BYTES == BG_NOALLOC_SCRATCH_BYTES, "keep BG_NOALLOC_SCRATCH_BYTES in step");
 
 static __device__ __align__(256) unsigned char g_scratch[SCRATCH_BYTES];
@@ -174,7 +174,6 @@ extern "C" bg_status bg_render_noalloc(const bg_scene* scene, const bg_camera* c
     w.queue[0] = reinterpret_cast<uint32_t*>(base + OFF_Q0);
     w.queue[1] = reinterpret_cast<uint32_t*>(base + OFF_Q1);
     w.cls_queue = reinterpret_cast<uint32_t*>(base + OFF_CLS);
-    w.done = reinterpret_cast<uint32_t*>(base + OFF_DONE);
     w.counters = reinterpret_cast<uint32_t*>(base + OFF_COUNTERS);
     w.ray_stats = reinterpret_cast<unsigned long long*>(base + OFF_RAYSTATS);
 
@@ -202,7 +201,7 @@ extern "C" bg_status bg_render_noalloc(const bg_scene* scene, const bg_camera* c
         return finish(reject(BG_ERR_CUDA, std::string("multiprocessor count: ") + cudaGetErrorString(e)));
     // fixed launch shape: bg_render's tuned shape and BG_TUNE_* settings belong to a bg_ctx, which
     // this entry point does not take
-    LaunchShape shape{dev_sms, 128, 8, 32};
+    LaunchShape shape{dev_sms, 128};
     Camera dc = camera_for(*cam);
     RenderParams rp{cam->width, cam->height, o->spp, o->max_depth, o->first_sample, o->rr_threshold, o->seed};
     rp = with_camera(rp, dc, o->spp);

@@ -5,16 +5,9 @@
 
 namespace bg {
 
-int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        uint32_t b, uint32_t* err, dim3 grid, cudaStream_t s) {
-    const dim3 sg = shade_grid(grid);
-    const GuideWave gw{};
-    k_shade<CLS_MISS><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<0, false, false, true, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<1, false, false, true, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<2, false, false, false, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    k_shade<3, false, false, false, true, true><<<sg, SHADE_BLOCK, 0, s>>>(sc, rp, film, wb, gw, b, err, nullptr);
-    return 5;
+int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t b, uint32_t* err,
+                        uint32_t blocks, const ShadeFork* fork, cudaStream_t s) {
+    return shade_launch<false, false, true, true, true>(sc, rp, wb, GuideWave{}, b, err, nullptr, sc.cls_mask, blocks, fork, s);
 }
 
 }  // namespace bg

@@ -22,8 +22,6 @@ namespace bg {
 // frame at 16 spp 94.6 / 96.0 ms (256: 3.63, 9.65, 95.0); the example scene, whose paths mostly
 // escape at once, loses 2%.  More barriers, between the parts of a vertex, cost more than they give.
 constexpr uint32_t SHADE_BLOCK = 512;
-// Grid of SHADE_BLOCK-thread blocks with the threads of `grid` blocks of 128.
-inline dim3 shade_grid(dim3 grid) { return dim3(grid.x * 128u / SHADE_BLOCK > 0 ? grid.x * 128u / SHADE_BLOCK : 1u); }
 
 // ================================================================ textures
 // Texture inputs at a hit whose material is textured (nullptr otherwise): the surface geometry
@@ -68,9 +66,14 @@ BG_D uint32_t st_k2(uint32_t st) { return st >> 24; }
 BG_D uint32_t st_set_k(uint32_t st, uint32_t k1, uint32_t k2) {
     return (st & 0xFFFFu) | (min(k1, 255u) << 16) | (min(k2, 255u) << 24);
 }
-enum : uint32_t { C_Q0 = 0, C_Q1 = 1, C_SHADOW = 2, C_DONE = 3, C_EXT_HEAD = 4, C_SH_HEAD = 5, C_CLS = 6 };
+// Queue counters.  Their resets ride along with kernels that precede the next use and follow the last
+// one: EXT_HEAD by generation and binning, the others by extension.
+enum : uint32_t { C_Q0 = 0, C_Q1 = 1, C_SHADOW = 2, C_EXT_HEAD = 4, C_SH_HEAD = 5, C_CLS = 6 };
 constexpr int NCLS = 5;          // material classes 0..3 (bg_material_type) + misses
 constexpr int CLS_MISS = 4;
+
+// A path's state at bounce 0: the camera sample made one get_1d and two get_2d calls.
+constexpr uint32_t CAMERA_STATE = (1u << 16) | (2u << 24);
 
 // Camera ray of (pixel, sample) into path slot i (PerspectiveCamera::generate_ray).
 BG_D void generate_one(const Camera& cam, const RenderParams& rp, const WaveBuffers& wb, uint32_t i, uint32_t pix,
@@ -83,16 +86,16 @@ BG_D void generate_one(const Camera& cam, const RenderParams& rp, const WaveBuff
     wb.ray_d[i] = make_float4(r.d.x, r.d.y, r.d.z, r.time);
     wb.pixel[i] = pix;
     wb.sample[i] = s;
-    wb.state[i] = st_set_k(0u, 1u, 2u);  // the camera sample made one get_1d and two get_2d calls
-    wb.beta[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    wb.L[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    wb.queue[0][i] = i;
+    wb.queue[0][i] = i;  // state, throughput and radiance start as CAMERA_STATE, 1 and 0 at bounce 0
 }
 
 BG_D void generate_paths(const Camera& cam, const RenderParams& rp, const WaveBuffers& wb, uint64_t item0,
                          uint32_t nitems, uint32_t first_sample) {
     const uint64_t npix = (uint64_t)rp.width * rp.height;
-    if (blockIdx.x == 0 && threadIdx.x == 0) wb.counters[C_Q0] = nitems;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        wb.counters[C_Q0] = nitems;
+        wb.counters[C_EXT_HEAD] = 0;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
         uint64_t item = item0 + i;
         generate_one(cam, rp, wb, i, pixel_of((uint32_t)(item % npix), rp.width, rp.height, rp.pixel_tiles),
@@ -428,6 +431,13 @@ BG_D void scatter_vertex(const Scene& sc, const RenderParams& rp, const WaveBuff
         wb.nee_beta[slot] = make_float4(beta.r, beta.g, beta.b, 0.0f);
         state |= ST_PENDING;
     }
+    // The ray behind the last vertex only looks for emission, which counts after specular bounces alone
+    // (path.rs:76-85): a matte, plastic or conductor vertex ends its path here.  Recording waves trace it
+    // for the training record's target.
+    if (GUIDABLE && !record && bounce + 1 >= rp.max_depth) {
+        out.finished = true;
+        return;
+    }
     V3 wo = -ray.d;
     BxSample bs;
     float p_b;  // BSDF pdf of the continuation (the training record's)
@@ -483,20 +493,19 @@ BG_D void scatter_vertex(const Scene& sc, const RenderParams& rp, const WaveBuff
 // Block-convergent tail of k_shade: queue compaction, shadow rays, records.
 // lrec: this lane's path resolved a visible light-sample record of its previous vertex.
 BG_D void finish_vertex(const WaveBuffers& wb, const GuideWave& gw, uint32_t bounce, uint32_t slot, bool cont,
-                        bool done_pending, const VertexOut& vo, uint32_t emit_n, RGB L_emit, bool record,
-                        uint32_t* err, bool lrec, BlockAppend<4>& append) {
-    uint32_t pos[4];
-    append({&wb.counters[(bounce + 1) & 1], &wb.counters[C_DONE], &wb.counters[C_SHADOW], &wb.counters[C_SHADOW]},
-           {cont, done_pending, vo.push_sh[0], vo.push_sh[1]}, pos);
+                        const VertexOut& vo, uint32_t emit_n, RGB L_emit, bool record, uint32_t* err, bool lrec,
+                        BlockAppend<3>& append) {
+    uint32_t pos[3];
+    append({&wb.counters[(bounce + 1) & 1], &wb.counters[C_SHADOW], &wb.counters[C_SHADOW]},
+           {cont, vo.push_sh[0], vo.push_sh[1]}, pos);
     if (cont) wb.queue[(bounce + 1) & 1][pos[0]] = slot;
-    if (done_pending) wb.done[pos[1]] = slot;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         if (vo.push_sh[k]) {
-            if (pos[2 + k] < wb.sh_capacity) {
-                wb.sh_o[pos[2 + k]] = vo.sh_o[k];
-                wb.sh_d[pos[2 + k]] = vo.sh_d[k];
-                wb.sh_ref[pos[2 + k]] = 2 * slot + (uint32_t)k;
+            if (pos[1 + k] < wb.sh_capacity) {
+                wb.sh_o[pos[1 + k]] = vo.sh_o[k];
+                wb.sh_d[pos[1 + k]] = vo.sh_d[k];
+                wb.sh_ref[pos[1 + k]] = 2 * slot + (uint32_t)k;
             } else {
                 atomicOr(err, ERR_QUEUE_OVERFLOW);
             }
@@ -508,153 +517,188 @@ BG_D void finish_vertex(const WaveBuffers& wb, const GuideWave& gw, uint32_t bou
     }
 }
 
-// Shades the paths of one material class (CLS = bg_material_type, or CLS_MISS for escaped rays).
-// In guided waves the matte / plastic / conductor classes read the network's mixture for their
+// What a block's unit of SHADE_BLOCK paths leaves for the block-wide tail.
+struct ShadeOut {
+    uint32_t slot = 0, emit_n = 0;
+    bool cont = false, lrec_emit = false;
+    VertexOut vo;
+    RGB L_emit = rgb(0.0f);
+};
+
+// Shades entry `i` of material class CLS's queue (CLS = bg_material_type, or CLS_MISS for escaped
+// rays).  In guided waves the matte / plastic / conductor classes read the network's mixture for their
 // queue position (inferred after binning, before this launch) and sample with it.
 // GWK: guiding support compiled in (records, mixtures); the plain wavefront uses GWK = false.
-// Minimum resident CTAs per SM the shade kernels are compiled for: 4 caps them at 128 registers
-// (the plastic and conductor classes would use 148 / 159).  Measured on the production scene at
-// 4 spp: shade 7.1 ms against 7.7 ms unconstrained; 5 and 6 CTAs gave 7.3 and 7.1 ms.
-#ifndef BG_SHADE_MINBLOCKS
-#define BG_SHADE_MINBLOCKS 4
-#endif
-// The guided variants hold the mixture views and eight more uniforms; they are compiled for
-// BG_GUIDED_SHADE_MINBLOCKS CTAs per SM (4: matte, plastic and conductor spill 36, 32, 44 bytes).
-#ifndef BG_GUIDED_SHADE_MINBLOCKS
-#define BG_GUIDED_SHADE_MINBLOCKS 4
-#endif
-template <int CLS, bool MULTI = false, bool GWK = false, bool TEX = false, bool INF = false, bool SHL = INF>
-__global__ void __launch_bounds__(SHADE_BLOCK, (GWK ? BG_GUIDED_SHADE_MINBLOCKS : BG_SHADE_MINBLOCKS) * 128 / SHADE_BLOCK) k_shade(Scene sc0, RenderParams rp0, FilmBuffers film0, WaveBuffers wb,
-                                               GuideWave gw, uint32_t bounce, uint32_t* err, const SceneRender* tab) {
+template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
+BG_D void shade_path(const Scene& sc0, const RenderParams& rp0, const WaveBuffers& wb, const GuideWave& gw,
+                     uint32_t bounce, const SceneRender* tab, uint32_t i, float* strat_col, ShadeOut& out) {
     constexpr bool GUIDABLE = CLS >= 0 && CLS <= 2;
-    const uint32_t n = wb.counters[C_CLS + CLS];
-    const uint32_t* q = wb.cls_queue + (size_t)CLS * wb.capacity;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    __shared__ float strat_su[CLS != CLS_MISS ? 8 * SU_STRIDE : 1];
     const bool record = GWK && (gw.flags & GW_RECORD) != 0;
     const bool guided = GWK && GUIDABLE && (gw.flags & GW_GUIDED);
-    __shared__ BlockAppend<4> append;
-    // block-uniform loop: the barriers below see every thread
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        __syncthreads();
-        uint32_t i = base + threadIdx.x;
-        bool active = i < n;
-        uint32_t slot = active ? q[i] : 0;
-        bool cont = false, done_pending = false, lrec_emit = false;
-        VertexOut vo;
-        uint32_t emit_n = 0;
-        RGB L_emit = rgb(0.0f);
-        if (active) {
-            const SceneRender* sr = MULTI ? tab + wb.scene_id[slot] : nullptr;
-            const Scene& sc = pick<MULTI>(sc0, MULTI ? &sr->sc : nullptr);
-            const RenderParams& rp = pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr);
-            const FilmBuffers& film = pick<MULTI>(film0, MULTI ? &sr->film : nullptr);
-            float4 ro = wb.ray_o[slot], rd = wb.ray_d[slot];
-            Ray ray = load_ray(ro, rd);
-            int prim = wb.hit[slot].x;
-            uint32_t state = wb.state[slot];
-            float4 b4 = wb.beta[slot];
-            RGB beta = rgb(b4.x, b4.y, b4.z);
-            float eta_scale = b4.w;
-            const float* su = nullptr;
-            if (CLS != CLS_MISS && rp.strat.dims > 0) {
-                float* col = strat_su + threadIdx.x;
-                strat_prefetch(rp.strat, wb.pixel[slot], wb.sample[slot], rp.seed, st_k1(state), st_k2(state), col);
-                su = col;
-            }
-            float4 l4 = wb.L[slot];
-            RGB L = apply_pending(wb, slot, rgb(l4.x, l4.y, l4.z), state, sc.nlights);
-            // the previous vertex's light-sample record: its shadow ray has been traced
-            if (record && (state & ST_LREC)) lrec_emit = wb.pending[2 * slot].w != 0.0f;
-            state &= ~(ST_PENDING | ST_LREC);
-            bool specular_bounce = (state & ST_SPECULAR) != 0;
-            Isect it;
-            bool hit = CLS != CLS_MISS && prim >= 0 && prim_isect(sc, prim, ray, &it);
-            const bool counted = bounce == 0 || specular_bounce;
-            const bool rec_open = record && (state & ST_REC_OPEN);
-            RGB le = hit && (counted || rec_open) ? emitted_radiance(sc, it, -ray.d) : rgb(0.0f);
-            // an escaped ray gathers the infinite light's radiance (path.rs:78-85)
-            if (CLS == CLS_MISS && prim < 0 && (counted || rec_open) && sc.inf) le = inf_radiance(sc, ray.d);
-            // The previous vertex's record closes here, with this emission as its direct target
-            // (which the estimator leaves to that vertex's next-event estimation unless counted).
-            if (record) state = close_record(gw, wb, slot, state, counted ? L + beta * le : L, beta * le);
-            if (counted) L = L + beta * le;
-            bool finished = !hit || bounce >= rp.max_depth;
-            if (!finished) {
-                // guided: the mixture inferred for this queue position (GW_CONT / GW_NEE place it)
-                const bool gv = guided && i < gw.cap;
-                const MixView mix{gv ? gw.raw + ((size_t)(GUIDABLE ? CLS : 0) * gw.cap + i) * GUIDE_MIX_HEAD : nullptr};
-                float ug[8];
-                if (gv) {
-                    const Rng grng{wb.pixel[slot], wb.sample[slot], rp.seed};
-                    grng.block(DIM_GUIDE0 + 8 * bounce, ug);
-                    grng.block(DIM_GUIDE0 + 8 * bounce + 4, ug + 4);
-                }
-                scatter_vertex<CLS, TEX, INF, SHL>(sc, rp, wb, gw, slot, bounce, ray, it, beta, eta_scale, state,
-                                                   gv ? &mix : nullptr, ug, record, vo, su);
-                finished = vo.finished;
-                cont = vo.cont;
-            }
-            wb.state[slot] = state;
-            wb.beta[slot] = make_float4(beta.r, beta.g, beta.b, eta_scale);
-            wb.L[slot] = make_float4(L.r, L.g, L.b, 0.0f);
-            if (finished) {
-                if (state & ST_PENDING) {
-                    done_pending = true;
-                } else {
-                    film_add(film, wb.pixel[slot], L);
-                    emit_n = rec_count(state);
-                    L_emit = L;
-                }
-            }
+    const uint32_t slot = wb.cls_queue[(size_t)CLS * wb.capacity + i];
+    out.slot = slot;
+    const SceneRender* sr = MULTI ? tab + wb.scene_id[slot] : nullptr;
+    const Scene& sc = pick<MULTI>(sc0, MULTI ? &sr->sc : nullptr);
+    const RenderParams& rp = pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr);
+    float4 ro = wb.ray_o[slot], rd = wb.ray_d[slot];
+    Ray ray = load_ray(ro, rd);
+    int prim = wb.hit[slot].x;
+    uint32_t state = bounce ? wb.state[slot] : CAMERA_STATE;
+    float4 b4 = bounce ? wb.beta[slot] : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    RGB beta = rgb(b4.x, b4.y, b4.z);
+    float eta_scale = b4.w;
+    const float* su = nullptr;
+    if (CLS != CLS_MISS && rp.strat.dims > 0) {
+        strat_prefetch(rp.strat, wb.pixel[slot], wb.sample[slot], rp.seed, st_k1(state), st_k2(state), strat_col);
+        su = strat_col;
+    }
+    float4 l4 = bounce ? wb.L[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    RGB L = apply_pending(wb, slot, rgb(l4.x, l4.y, l4.z), state, sc.nlights);
+    // the previous vertex's light-sample record: its shadow ray has been traced
+    if (record && (state & ST_LREC)) out.lrec_emit = wb.pending[2 * slot].w != 0.0f;
+    state &= ~(ST_PENDING | ST_LREC);
+    bool specular_bounce = (state & ST_SPECULAR) != 0;
+    Isect it;
+    bool hit = CLS != CLS_MISS && prim >= 0 && prim_isect(sc, prim, ray, &it);
+    const bool counted = bounce == 0 || specular_bounce;
+    const bool rec_open = record && (state & ST_REC_OPEN);
+    RGB le = hit && (counted || rec_open) ? emitted_radiance(sc, it, -ray.d) : rgb(0.0f);
+    // an escaped ray gathers the infinite light's radiance (path.rs:78-85)
+    if (CLS == CLS_MISS && prim < 0 && (counted || rec_open) && sc.inf) le = inf_radiance(sc, ray.d);
+    // The previous vertex's record closes here, with this emission as its direct target
+    // (which the estimator leaves to that vertex's next-event estimation unless counted).
+    if (record) state = close_record(gw, wb, slot, state, counted ? L + beta * le : L, beta * le);
+    if (counted) L = L + beta * le;
+    bool finished = !hit || bounce >= rp.max_depth;
+    if (CLS != CLS_MISS && !finished) {
+        // guided: the mixture inferred for this queue position (GW_CONT / GW_NEE place it)
+        const bool gv = guided && i < gw.cap;
+        const MixView mix{gv ? gw.raw + ((size_t)(GUIDABLE ? CLS : 0) * gw.cap + i) * GUIDE_MIX_HEAD : nullptr};
+        float ug[8];
+        if (gv) {
+            const Rng grng{wb.pixel[slot], wb.sample[slot], rp.seed};
+            grng.block(DIM_GUIDE0 + 8 * bounce, ug);
+            grng.block(DIM_GUIDE0 + 8 * bounce + 4, ug + 4);
         }
-        finish_vertex(wb, gw, bounce, slot, cont, done_pending, vo, emit_n, L_emit, record, err, lrec_emit, append);
+        scatter_vertex<CLS, TEX, INF, SHL>(sc, rp, wb, gw, slot, bounce, ray, it, beta, eta_scale, state,
+                                           gv ? &mix : nullptr, ug, record, out.vo, su);
+        finished = out.vo.finished;
+        out.cont = out.vo.cont;
+    }
+    // a finished path's radiance stays in L (and its last vertex's light contribution in `pending`)
+    // until the wave's paths are added to the film
+    wb.state[slot] = state;
+    wb.L[slot] = make_float4(L.r, L.g, L.b, 0.0f);
+    if (!finished) wb.beta[slot] = make_float4(beta.r, beta.g, beta.b, eta_scale);
+    else if (GWK && !(state & ST_PENDING)) {
+        out.emit_n = rec_count(state);
+        out.L_emit = L;
+    }
+}
+
+// A block's unit: entries base .. base + SHADE_BLOCK - 1 of class CLS's queue of n.
+template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
+BG_D void shade_unit(const Scene& sc0, const RenderParams& rp0, const WaveBuffers& wb, const GuideWave& gw,
+                     uint32_t bounce, uint32_t* err, const SceneRender* tab, uint32_t base, uint32_t n, float* strat_col,
+                     BlockAppend<3>& append) {
+    const uint32_t i = base + threadIdx.x;
+    ShadeOut out;
+    if (i < n) shade_path<CLS, MULTI, GWK, TEX, INF, SHL>(sc0, rp0, wb, gw, bounce, tab, i, strat_col, out);
+    finish_vertex(wb, gw, bounce, out.slot, out.cont, out.vo, out.emit_n, out.L_emit,
+                  GWK && (gw.flags & GW_RECORD) != 0, err, out.lrec_emit, append);
+}
+
+// Shades a bounce's paths of material class CLS.  One block of 512 threads per SM: 128 registers.
+template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
+__global__ void __launch_bounds__(SHADE_BLOCK, 1) k_shade(Scene sc0, RenderParams rp0, WaveBuffers wb, GuideWave gw,
+                                                          uint32_t bounce, uint32_t* err, const SceneRender* tab) {
+    __shared__ float strat_su[CLS != CLS_MISS ? 8 * SU_STRIDE : SU_STRIDE];
+    __shared__ BlockAppend<3> append;
+    const uint32_t n = wb.counters[C_CLS + CLS];
+    for (uint32_t base = blockIdx.x * SHADE_BLOCK; base < n; base += gridDim.x * SHADE_BLOCK) {
+        __syncthreads();
+        shade_unit<CLS, MULTI, GWK, TEX, INF, SHL>(sc0, rp0, wb, gw, bounce, err, tab, base, n, strat_su + threadIdx.x,
+                                                   append);
     }
 }
 
 // Streams of one bounce's class kernels.  The classes share no data a kernel of another class
 // reads (each shades its own queue's paths, writes only those paths' slots and appends to the next
-// queues and the training pool with atomics), so with a fork they run side by side: matte (the
-// largest class) on the launching stream, plastic, conductor, dielectric and the misses on the
-// fork's streams, which first wait for everything already on `s`; shade_join makes `s` wait for
-// them again.
+// queues and the training pool with atomics), so with a fork they run side by side: the first class the
+// scene has on the launching stream, every other one on a fork stream, which first waits for everything
+// already on `s`, and the misses behind the last class; shade_join makes `s` wait for them again.
+// Only the classes of `mask` (Scene::cls_mask) take launches and event calls: all five of every scene
+// were 5 launches and 13 event calls a bounce, most of a small film's time on the host.
 struct ClassStreams {
     cudaStream_t st[5];  // by class: matte, plastic, conductor, dielectric, misses
+    int used = 0;        // fork streams in use
 };
-inline ClassStreams shade_fork(cudaStream_t s, const ShadeFork* fork) {
+inline ClassStreams shade_fork(cudaStream_t s, const ShadeFork* fork, uint32_t mask) {
     ClassStreams cs{{s, s, s, s, s}};
-    if (fork) {
-        cudaEventRecord(fork->fork, s);
-        for (int k = 0; k < 4; ++k) {
-            cudaStreamWaitEvent(fork->aux[k], fork->fork, 0);
-            cs.st[1 + k] = fork->aux[k];
+    if (!fork) return cs;
+    cudaStream_t last = s;
+    bool first = true;
+    for (int c = 0; c < 4; ++c) {
+        if (!((mask >> c) & 1u)) continue;
+        if (!first) {
+            if (cs.used == 0) cudaEventRecord(fork->fork, s);
+            cudaStreamWaitEvent(fork->aux[cs.used], fork->fork, 0);
+            last = fork->aux[cs.used++];
         }
+        first = false;
+        cs.st[c] = last;
     }
+    cs.st[4] = last;
     return cs;
 }
-inline void shade_join(cudaStream_t s, const ShadeFork* fork) {
-    if (!fork) return;
-    for (int k = 0; k < 4; ++k) {
+inline void shade_join(cudaStream_t s, const ShadeFork* fork, const ClassStreams& cs) {
+    for (int k = 0; k < cs.used; ++k) {
         cudaEventRecord(fork->join[k], fork->aux[k]);
         cudaStreamWaitEvent(s, fork->join[k], 0);
     }
 }
 
-// Single-scene shade launches for scenes with emitting spheres or quadrics (bg_shade_shapes.cu).
-int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s);
-// Shade launches of one bounce (the five material classes, misses included); with `fork` the
-// classes run on parallel streams, joined back into `s` before returning.
-int launch_shade_plain(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                       uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s,
-                       const ShadeFork* fork = nullptr);
-int launch_shade_guided(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                        const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s,
-                        const ShadeFork* fork = nullptr);
-// The guided launches of scenes with textures or an infinite light (bg_shade_guided_full.cu).
-int launch_shade_guided_full(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
-                             const GuideWave& gw, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s, const ShadeFork* fork = nullptr);
-// full: the variants that handle textured scenes and infinite lights (checked per path's scene).
-int launch_shade_batch(const SceneRender* tab, const WaveBuffers& wb, uint32_t bounce, uint32_t* err, dim3 grid, cudaStream_t s, bool full);
+// A bounce's class kernels (of the classes in `mask`, and the misses); the texture code is compiled into
+// the classes that have textures.
+template <bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
+inline int shade_launch(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, const GuideWave& gw, uint32_t b,
+                        uint32_t* err, const SceneRender* tab, uint32_t mask, uint32_t blocks, const ShadeFork* fork,
+                        cudaStream_t s) {
+    const ClassStreams cs = shade_fork(s, fork, mask);
+    const cudaStream_t* st = cs.st;
+    int n = 1;
+#define BG_CLASS(C, T, I, S)                                                                                        \
+    if ((mask >> C) & 1u) {                                                                                         \
+        k_shade<C, MULTI, GWK, T, I, S><<<blocks, SHADE_BLOCK, 0, st[C]>>>(sc, rp, wb, gw, b, err, tab);             \
+        ++n;                                                                                                        \
+    }
+    BG_CLASS(0, TEX, INF, SHL)
+    BG_CLASS(1, TEX, INF, SHL)
+    BG_CLASS(2, false, INF, SHL)
+    BG_CLASS(3, false, false, false)
+#undef BG_CLASS
+    k_shade<CLS_MISS, MULTI, GWK, false, false, false><<<blocks, SHADE_BLOCK, 0, st[4]>>>(sc, rp, wb, gw, b, err, tab);
+    shade_join(s, fork, cs);
+    return n;
+}
+
+// The shade launches of a bounce, each returning the kernels launched; with `fork` the classes run on
+// parallel streams, joined back into `s` before returning.
+// Plain single-scene waves (bg_shade_plain.cu); scenes with emitting spheres or quadrics
+// (bg_shade_shapes.cu).
+int launch_shade_plain(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t bounce, uint32_t* err,
+                       uint32_t blocks, const ShadeFork* fork, cudaStream_t s);
+int launch_shade_shapes(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t bounce, uint32_t* err,
+                        uint32_t blocks, const ShadeFork* fork, cudaStream_t s);
+// Guided waves (bg_shade_aux.cu), and those of scenes with textures or general lights
+// (bg_shade_guided_full.cu).
+int launch_shade_guided(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, const GuideWave& gw,
+                        uint32_t bounce, uint32_t* err, uint32_t blocks, const ShadeFork* fork, cudaStream_t s);
+int launch_shade_guided_full(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, const GuideWave& gw,
+                             uint32_t bounce, uint32_t* err, uint32_t blocks, const ShadeFork* fork, cudaStream_t s);
+// Batch waves.  full: the variants that handle textured scenes and infinite lights (checked per
+// path's scene).
+int launch_shade_batch(const SceneRender* tab, const WaveBuffers& wb, uint32_t bounce, uint32_t* err, uint32_t mask,
+                       uint32_t blocks, const ShadeFork* fork, cudaStream_t s, bool full);
 
 }  // namespace bg
