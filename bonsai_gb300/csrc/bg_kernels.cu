@@ -7,9 +7,7 @@
 // Traversal stages pull 32-ray batches per warp from an atomic head (dynamic load balance);
 // queues are compacted with warp ballot + popc + one atomic per warp.
 //
-// Megakernel (both modes, reference-layout BVH): one thread per (pixel, sample) runs
-// PathIntegrator::radiance end to end; it is the REF_COMPAT path and a cross-check of the
-// wavefront in PBRT mode.
+// Renders over the reference layout (REF_COMPAT, and PBRT as a cross-check) run per path: bg_mega.cu.
 #include "bg_guide.cuh"
 #include "bg_guide_kernels.h"
 #include "bg_kernels.h"
@@ -97,95 +95,6 @@ void launch_trace(const Scene& sc, bool ref_layout, bool any, const bg_ray* rays
         else BG_TRACE(8, false);
     }
 #undef BG_TRACE
-}
-
-// ================================================================ megakernel (reference layout)
-// `rd0`: the camera ray's differentials (textured scenes), which the path keeps in REF mode (the
-// ray never re-spawns, F1) and only has at the first hit in PBRT mode.
-template <bool REF>
-BG_D RGB radiance_ref(const Scene& sc, Ray ray, const Rng& rng, uint32_t max_depth, float rr_threshold,
-                      uint32_t* err, const RayDiff* rd0, const StratParams& sp) {
-    SamplerCalls calls{sp, REF, rng.pixel, rng.sample, rng.seed, 1u, 2u};  // after the camera sample
-    RGB out = rgb(0.0f), beta = rgb(1.0f);
-    bool specular_bounce = false;
-    float eta_scale = 1.0f;
-    for (uint32_t bounces = 0;; ++bounces) {
-        Ray traced = ray;
-        int prim = ref_traverse<false>(sc, ray, err, nullptr);  // sets ray.t_max to the hit
-        bool hit = prim >= 0;
-        Isect it;
-        if (hit) hit = prim_isect(sc, prim, traced, &it);
-        if (bounces == 0 || specular_bounce) {
-            if (hit) out = out + beta * emitted_radiance(sc, it, -ray.d);
-            else if (prim < 0) out = out + beta * escaped_radiance(sc, ray.d);
-        }
-        if (!hit || bounces >= max_depth) break;
-        TexPoint tp;
-        BSDF bsdf = make_bsdf<-1, REF>(sc, it, tex_point(sc, it, traced, (REF || bounces == 0) ? rd0 : nullptr, &tp));
-        const uint32_t base = DIM_BOUNCE0 + DIMS_PER_BOUNCE * bounces;
-        float u[8];
-        rng.block(base, u);
-        rng.block(base + 4, u + 4);
-        if (bsdf.num_components(BSDF_ALL & ~BSDF_SPECULAR) > 0 && sc.nlights > 0) {
-            calls.get_1d(u[BD_LIGHT]);
-            calls.get_2d(u[BD_ULIGHT], u[BD_ULIGHT + 1]);
-            calls.get_2d(u[BD_USCAT], u[BD_USCAT + 1]);
-            float count = (float)sc.nlights;
-            uint32_t li = (uint32_t)rmin(u[BD_LIGHT] * count, count - 1.0f);
-            float lpdf = 1.0f / count;
-            RGB ld = estimate_direct_mk<REF, 1>(sc, it, bsdf, sc.light_prims[li], u[BD_USCAT], u[BD_USCAT + 1],
-                                              u[BD_ULIGHT], u[BD_ULIGHT + 1], err);
-            out = out + beta * (ld / lpdf);
-        }
-        V3 wo = -ray.d;
-        calls.get_2d(u[BD_BSDF], u[BD_BSDF + 1]);
-        BxSample bs = bsdf.sample<REF>(wo, u[BD_BSDF], u[BD_BSDF + 1], BSDF_ALL);
-        if (is_black(bs.f) || bs.pdf == 0.0f) break;
-        beta = beta * (bs.f * abs_dot(bs.wi, it.ns) / bs.pdf);
-        specular_bounce = (bs.stype & BSDF_SPECULAR) != 0;
-        if ((bs.stype & BSDF_SPECULAR) && (bs.stype & BSDF_TRANSMISSION)) {
-            float eta = bsdf.eta;
-            eta_scale *= dot(wo, it.n) > 0.0f ? eta * eta : 1.0f / (eta * eta);
-        }
-        // F1: REF re-intersects the same ray (t_max already at this hit); PBRT moves on
-        if (!REF) ray = spawn_ray(it.p, it.p_err, it.n, it.time, bs.wi, false);
-        RGB rr_beta = beta * eta_scale;
-        if (max_value(rr_beta) < rr_threshold && bounces > 3) {
-            calls.get_1d(u[BD_RR]);
-            float q = rmax(1.0f - max_value(rr_beta), 0.5f);
-            if (u[BD_RR] < q) break;
-            beta = beta / (1.0f - q);
-        }
-    }
-    return out;
-}
-
-template <bool REF>
-__global__ void __launch_bounds__(128) k_megakernel(Scene sc, Camera cam, RenderParams rp, FilmBuffers film,
-                                                    uint32_t* err) {
-    const uint64_t npix = (uint64_t)rp.width * rp.height;
-    const uint64_t total = npix * rp.spp;
-    for (uint64_t item = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; item < total;
-         item += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t pix = (uint32_t)(item % npix);
-        uint32_t s = rp.first_sample + (uint32_t)(item / npix);
-        Rng rng{pix, s, rp.seed};
-        const CameraUs cu = camera_us(rp.strat, REF, rng, cam.lens_radius > 0.0f);
-        float fx = (float)(pix % rp.width) + cu.fx, fy = (float)(pix / rp.width) + cu.fy;
-        Ray ray = camera_ray(cam, fx, fy, cu.time, cu.lx, cu.ly);
-        RayDiff rd;
-        if (sc.ntex) rd = camera_diff(cam, fx, fy, ray, rp.diff_scale, cu.lx, cu.ly);
-        RGB L = radiance_ref<REF>(sc, ray, rng, rp.max_depth, rp.rr_threshold, err, sc.ntex ? &rd : nullptr,
-                                  rp.strat);
-        film_add(film, pix, L);
-    }
-}
-
-void launch_megakernel(bool ref_compat, const Scene& sc, const Camera& cam, const RenderParams& rp,
-                       const FilmBuffers& film, uint32_t* err, const LaunchShape& ls, cudaStream_t s) {
-    dim3 grid(ls.sms * 8), block(128);
-    if (ref_compat) k_megakernel<true><<<grid, block, 0, s>>>(sc, cam, rp, film, err);
-    else k_megakernel<false><<<grid, block, 0, s>>>(sc, cam, rp, film, err);
 }
 
 // Batch: item -> scene by binary search over the scenes' first items, then as above.

@@ -43,111 +43,6 @@ BG_D bool ref_slab(const RefNode& nd, const Ray& ray, V3 inv, const int neg[3]) 
     return (t_min < ray.t_max) && (t_max > 0.0f);
 }
 
-// Primitive test against the current t_max; updates ray.t_max on a closest hit.
-BG_D bool prim_hit(const Scene& sc, uint32_t prim, const TriRay& tr, Ray& ray, bool closest) {
-    if (prim < sc.ntri) {
-        V3 p0, p1, p2;
-        load_tri(sc, prim, &p0, &p1, &p2);
-        TriHit h;
-        if (!tri_test(tr, ray.t_max, p0, p1, p2, &h)) return false;
-        if (closest) ray.t_max = h.t;
-        return true;
-    }
-    if (prim < sc.ntri + sc.nsph) {
-        SphHit h;
-        if (!sphere_test(sc.sph[prim - sc.ntri], ray, ray.t_max, closest ? &h : nullptr)) return false;
-        if (closest) ray.t_max = h.t;
-        return true;
-    }
-    float t;
-    if (!quadric_hit(sc.quads + QUADRIC_F4 * (prim - sc.ntri - sc.nsph), ray, ray.t_max, &t, nullptr)) return false;
-    if (closest) ray.t_max = t;
-    return true;
-}
-
-// BVH::intersect: returns the hit prim (or -1) and leaves the hit distance in ray.t_max.
-// counters (optional): [0] node visits, [1] primitive tests.
-template <bool ANY>
-BG_D int ref_traverse(const Scene& sc, Ray& ray, uint32_t* err, unsigned long long* counters) {
-    if (sc.ref_nnodes == 0) return -1;
-    V3 inv = v3(1.0f / ray.d.x, 1.0f / ray.d.y, 1.0f / ray.d.z);
-    int neg[3] = {inv.x < 0.0f, inv.y < 0.0f, inv.z < 0.0f};
-    TriRay tr = make_tri_ray(ray);
-    uint32_t stack[TRAVERSAL_STACK];
-    int sp = 0;
-    uint32_t cur = 0;
-    int hit = -1;
-    unsigned long long visits = 0, tests = 0;
-    for (;;) {
-        if (cur >= sc.ref_nnodes) {
-            atomicOr(err, ERR_BAD_NODE);
-            break;
-        }
-        const RefNode nd = sc.ref_nodes[cur];
-        ++visits;
-        uint32_t count = nd.count_axis >> 2;
-        if (ref_slab(nd, ray, inv, neg)) {
-            if (count > 0) {
-                for (uint32_t i = 0; i < count; ++i) {
-                    uint32_t prim = sc.ref_order[nd.offset + i];
-                    ++tests;
-                    if (prim_hit(sc, prim, tr, ray, !ANY)) {
-                        hit = (int)prim;
-                        if (ANY) goto done;
-                    }
-                }
-                if (sp == 0) break;
-                cur = stack[--sp];
-            } else {
-                if (sp >= TRAVERSAL_STACK) {
-                    atomicOr(err, ERR_STACK_OVERFLOW);
-                    hit = -1;
-                    break;
-                }
-                if (neg[nd.count_axis & 3]) {
-                    stack[sp++] = cur + 1;
-                    cur = nd.offset;
-                } else {
-                    stack[sp++] = nd.offset;
-                    cur = cur + 1;
-                }
-            }
-        } else {
-            if (sp == 0) break;
-            cur = stack[--sp];
-        }
-    }
-done:
-    if (counters) {
-        atomicAdd(&counters[0], visits);
-        atomicAdd(&counters[1], tests);
-    }
-    return hit;
-}
-
-// ---------------------------------------------------------------- 2-wide layout
-struct FastRay {
-    V3 inv, oi;  // 1/d and o/d (so t = fma(b, inv, -oi))
-};
-BG_D float safe_dir(float d) { return fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d); }
-BG_D FastRay make_fast_ray(const Ray& r) {
-    FastRay f;
-    f.inv = v3(1.0f / safe_dir(r.d.x), 1.0f / safe_dir(r.d.y), 1.0f / safe_dir(r.d.z));
-    f.oi = v3(r.o.x * f.inv.x, r.o.y * f.inv.y, r.o.z * f.inv.z);
-    return f;
-}
-// Returns entry distance, or +inf on a miss (the box must start before t_max and end after 0).
-BG_D float box_enter(float lox, float hix, float loy, float hiy, float loz, float hiz, const FastRay& f,
-                     float t_max) {
-    const float k = 1.0f + 2.0f * gamma(3.0f);
-    float tx0 = fmaf(lox, f.inv.x, -f.oi.x), tx1 = fmaf(hix, f.inv.x, -f.oi.x);
-    float ty0 = fmaf(loy, f.inv.y, -f.oi.y), ty1 = fmaf(hiy, f.inv.y, -f.oi.y);
-    float tz0 = fmaf(loz, f.inv.z, -f.oi.z), tz1 = fmaf(hiz, f.inv.z, -f.oi.z);
-    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.0f));
-    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1)) * k;
-    return (tn <= tf && tn < t_max) ? tn : INFINITY;
-}
-
 // sphere_test's hit and distance, bit for bit, without its interval arithmetic where that decides
 // nothing.  The roots' values (EF::v) never depend on the intervals, and an EFloat's value lies
 // inside its interval, so a root beyond t_max or a far root <= 0 rejects as it stands; the other
@@ -222,6 +117,114 @@ BG_D bool sphere_hit(float4 s, const Ray& ray, float* t) {
     const bool hit = sphere_test(s, ray, ray.t_max, &h);
     *t = h.t;
     return hit;
+}
+
+// Primitive test against the current t_max; updates ray.t_max on a closest hit.  INTERVALS: spheres
+// with their EFloat intervals, as the reference (the ray queries over its layout), else sphere_hit.
+template <bool INTERVALS>
+BG_D bool prim_hit(const Scene& sc, uint32_t prim, const TriRay& tr, Ray& ray, bool closest) {
+    if (prim < sc.ntri) {
+        V3 p0, p1, p2;
+        load_tri(sc, prim, &p0, &p1, &p2);
+        TriHit h;
+        if (!tri_test(tr, ray.t_max, p0, p1, p2, &h)) return false;
+        if (closest) ray.t_max = h.t;
+        return true;
+    }
+    if (prim < sc.ntri + sc.nsph) {
+        SphHit h;
+        if (INTERVALS ? !sphere_test(sc.sph[prim - sc.ntri], ray, ray.t_max, &h) : !sphere_hit(sc.sph[prim - sc.ntri], ray, &h.t))
+            return false;
+        if (closest) ray.t_max = h.t;
+        return true;
+    }
+    float t;
+    if (!quadric_hit(sc.quads + QUADRIC_F4 * (prim - sc.ntri - sc.nsph), ray, ray.t_max, &t, nullptr)) return false;
+    if (closest) ray.t_max = t;
+    return true;
+}
+
+// BVH::intersect: returns the hit prim (or -1) and leaves the hit distance in ray.t_max.
+// counters (optional): [0] node visits, [1] primitive tests.
+template <bool ANY, bool INTERVALS = true>
+BG_D int ref_traverse(const Scene& sc, Ray& ray, uint32_t* err, unsigned long long* counters) {
+    if (sc.ref_nnodes == 0) return -1;
+    V3 inv = v3(1.0f / ray.d.x, 1.0f / ray.d.y, 1.0f / ray.d.z);
+    int neg[3] = {inv.x < 0.0f, inv.y < 0.0f, inv.z < 0.0f};
+    TriRay tr = make_tri_ray(ray);
+    uint32_t stack[TRAVERSAL_STACK];
+    int sp = 0;
+    uint32_t cur = 0;
+    int hit = -1;
+    unsigned long long visits = 0, tests = 0;
+    for (;;) {
+        if (cur >= sc.ref_nnodes) {
+            atomicOr(err, ERR_BAD_NODE);
+            break;
+        }
+        const RefNode nd = sc.ref_nodes[cur];
+        ++visits;
+        uint32_t count = nd.count_axis >> 2;
+        if (ref_slab(nd, ray, inv, neg)) {
+            if (count > 0) {
+                for (uint32_t i = 0; i < count; ++i) {
+                    uint32_t prim = sc.ref_order[nd.offset + i];
+                    ++tests;
+                    if (prim_hit<INTERVALS>(sc, prim, tr, ray, !ANY)) {
+                        hit = (int)prim;
+                        if (ANY) goto done;
+                    }
+                }
+                if (sp == 0) break;
+                cur = stack[--sp];
+            } else {
+                if (sp >= TRAVERSAL_STACK) {
+                    atomicOr(err, ERR_STACK_OVERFLOW);
+                    hit = -1;
+                    break;
+                }
+                if (neg[nd.count_axis & 3]) {
+                    stack[sp++] = cur + 1;
+                    cur = nd.offset;
+                } else {
+                    stack[sp++] = nd.offset;
+                    cur = cur + 1;
+                }
+            }
+        } else {
+            if (sp == 0) break;
+            cur = stack[--sp];
+        }
+    }
+done:
+    if (counters) {
+        atomicAdd(&counters[0], visits);
+        atomicAdd(&counters[1], tests);
+    }
+    return hit;
+}
+
+// ---------------------------------------------------------------- 2-wide layout
+struct FastRay {
+    V3 inv, oi;  // 1/d and o/d (so t = fma(b, inv, -oi))
+};
+BG_D float safe_dir(float d) { return fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d); }
+BG_D FastRay make_fast_ray(const Ray& r) {
+    FastRay f;
+    f.inv = v3(1.0f / safe_dir(r.d.x), 1.0f / safe_dir(r.d.y), 1.0f / safe_dir(r.d.z));
+    f.oi = v3(r.o.x * f.inv.x, r.o.y * f.inv.y, r.o.z * f.inv.z);
+    return f;
+}
+// Returns entry distance, or +inf on a miss (the box must start before t_max and end after 0).
+BG_D float box_enter(float lox, float hix, float loy, float hiy, float loz, float hiz, const FastRay& f,
+                     float t_max) {
+    const float k = 1.0f + 2.0f * gamma(3.0f);
+    float tx0 = fmaf(lox, f.inv.x, -f.oi.x), tx1 = fmaf(hix, f.inv.x, -f.oi.x);
+    float ty0 = fmaf(loy, f.inv.y, -f.oi.y), ty1 = fmaf(hiy, f.inv.y, -f.oi.y);
+    float tz0 = fmaf(loz, f.inv.z, -f.oi.z), tz1 = fmaf(hiz, f.inv.z, -f.oi.z);
+    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.0f));
+    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1)) * k;
+    return (tn <= tf && tn < t_max) ? tn : INFINITY;
 }
 
 // Leaf slot: triangle = (p0, id) (p1, -) (p2, -); sphere = (center, id | SPHERE_BIT) (radius, -, -, -);

@@ -44,3 +44,21 @@ def test_smallest_films(gpu_ctx, size):
     assert r.stats.error_word == 0
     _, _, n = G.PathIntegrator.moments(gpu_ctx, w, h)
     assert (n == 1).all()
+
+
+@pytest.mark.parametrize("mode", [A.BG_MODE_REF_COMPAT, A.BG_MODE_PBRT])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (33, 1, 1), (1023, 1, 1), (1025, 1, 3), (400, 401, 1)])
+def test_per_path_kernel_films(gpu_ctx, mode, w, h, spp):
+    """Reference layout: fewer paths than a block, than the grid, and more (threads start further
+    paths).  Every sample reaches the film once, and the film equals the oracle's: same paths and
+    operations without contraction, so all but a few channels are equal to 1e-5 (transcendental
+    functions of the two machines differ in their last bits)."""
+    import oracle as O
+    sd = S.cornell(w, h, spp=spp)
+    sc = G.Scene(gpu_ctx, sd, A.BG_BVH_REFERENCE)
+    r = G.PathIntegrator(sd.camera, spp, 5, mode=mode).render(sc)
+    assert r.stats.error_word == 0
+    _, _, n = G.PathIntegrator.moments(gpu_ctx, w, h)
+    assert (n == spp).all()
+    ref = O.OracleScene(sd, fixed_bvh=False).render(mode)["rgb"]
+    assert np.mean(np.abs(r.rgb - ref) <= 1e-5 * (1.0 + np.abs(ref))) >= 0.99
