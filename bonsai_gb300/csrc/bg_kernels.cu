@@ -115,7 +115,8 @@ __global__ void k_generate_batch(const SceneRender* tab, uint32_t nscenes, WaveB
         const SceneRender& sr = tab[lo];
         const uint64_t local = item - sr.item0;
         const uint64_t npix = (uint64_t)sr.rp.width * sr.rp.height;
-        generate_one(sr.cam, sr.rp, wb, i, (uint32_t)(local % npix), sr.rp.first_sample + (uint32_t)(local / npix));
+        const uint32_t pix = (uint32_t)(local % npix);
+        generate_one(sr.cam, sr.rp, wb, i, {pix % sr.rp.width, pix / sr.rp.width}, sr.rp.first_sample + (uint32_t)(local / npix));
         wb.scene_id[i] = lo;
     }
 }
@@ -450,7 +451,7 @@ static int launch_bounces(const Scene& sc, const RenderParams& rp, const WaveBuf
     int launches = 0;
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     const dim3 bin_grid(ls.sms * 4);  // 2048 threads per SM
-    const uint32_t shade_blocks = 2 * (uint32_t)ls.sms;
+    const uint32_t shade_blocks = 2 * (uint32_t)ls.sms;  // one resident, one to even out the tail
     const GuideWave gw = gwp ? *gwp : GuideWave{};
     const bool guided = (gw.flags & GW_GUIDED) != 0;
     for (uint32_t b = 0; b <= rp.max_depth; ++b) {

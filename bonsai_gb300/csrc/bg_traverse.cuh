@@ -333,6 +333,17 @@ BG_D int bvh2_traverse(const Scene& sc, Ray& ray, uint32_t* err, int skip = -1) 
 // idle the warp fetches that many new rays with one atomic (Aila & Laine, HPG 2009, dynamic
 // fetch).  refill = 32 fetches only when the whole warp is idle.  Src supplies rays and takes
 // results: Ray load(uint32_t i, int* skip), void store(uint32_t i, int prim, float t).
+//
+// Few rays are spread over all the warps of the grid, down to one ray per warp: a warp takes a step for
+// each kind of work that any of its lanes has, so a warp of few rays finishes them sooner, and the
+// warps of a short queue fit the GPU side by side anyway.  Against full warps: 1021 rays, closest and
+// any hit, 206 -> 181 us a call pair; 67 x 49 preview 427 -> 409 us; uneven batch 3.69 -> 3.47 ms; at least
+// two or four rays per warp give less of it, long queues are not touched.
+BG_D uint32_t rays_per_warp(uint32_t n) {
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    return min(32u, (n + nwarps - 1) / nwarps);
+}
+
 template <bool ANY, class Src>
 BG_D void traverse_queue(const Scene& sc, uint32_t n, uint32_t* head, Src& src, uint32_t* err, int refill) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -342,7 +353,7 @@ BG_D void traverse_queue(const Scene& sc, uint32_t n, uint32_t* head, Src& src, 
     TriRay tr;
     int sp = 0, node = -2, hit = -1, skip = -1, leaf_first = 0, leaf_count = 0;
     uint32_t idx = 0;
-    bool busy = false, exhausted = false;
+    bool busy = false, exhausted = lane >= rays_per_warp(n);
     for (;;) {
         // refill idle lanes
         const unsigned idle = __ballot_sync(0xffffffffu, !busy && !exhausted);
@@ -675,7 +686,7 @@ BG_D void traverse_queue8(const Scene& sc, uint32_t n, uint32_t* head, Src& src,
     uint2 ngroup = make_uint2(0, 0), tgroup = make_uint2(0, 0);
     int sp = 0, hit = -1, skip = -1;
     uint32_t idx = 0;
-    bool busy = false, exhausted = false;
+    bool busy = false, exhausted = lane >= rays_per_warp(n);
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !busy && !exhausted);
         const int nidle = __popc(idle);

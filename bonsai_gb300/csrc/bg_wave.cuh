@@ -15,13 +15,19 @@
 
 namespace bg {
 
-// Threads per block of the shade kernels, whose warps go through the code side by side (a barrier at
+// Threads per block of the shade kernels (shade_block), whose warps go through the code side by side (a barrier at
 // every path): their code is 100 to 550 KB, far beyond the instruction caches, and a line fetched
 // for one warp serves the others of the block only while they are near it.  One block of 512 per SM
 // against four of 128: textured room 3.43 / 3.99 ms, guided slit room 9.34 / 10.04 ms, production
 // frame at 16 spp 94.6 / 96.0 ms (256: 3.63, 9.65, 95.0); the example scene, whose paths mostly
 // escape at once, loses 2%.  More barriers, between the parts of a vertex, cost more than they give.
-constexpr uint32_t SHADE_BLOCK = 512;
+// The guided variants and those with textures but no infinite light take 768 threads (80 registers): they
+// wait longer per instruction (guided slit room 8.89 -> 8.75 ms, textured room 3.20 -> 3.04; the plain
+// variants lose 1 to 2% to it: Cornell box 1.74 -> 1.77, example scene 4.98 -> 5.04).
+constexpr uint32_t SHADE_BLOCK_MAX = 768;
+constexpr __host__ __device__ uint32_t shade_block(bool guided, bool textured, bool infinite) {
+    return guided || (textured && !infinite) ? SHADE_BLOCK_MAX : 512u;
+}
 
 // ================================================================ textures
 // Texture inputs at a hit whose material is textured (nullptr otherwise): the surface geometry
@@ -76,11 +82,12 @@ constexpr int CLS_MISS = 4;
 constexpr uint32_t CAMERA_STATE = (1u << 16) | (2u << 24);
 
 // Camera ray of (pixel, sample) into path slot i (PerspectiveCamera::generate_ray).
-BG_D void generate_one(const Camera& cam, const RenderParams& rp, const WaveBuffers& wb, uint32_t i, uint32_t pix,
+BG_D void generate_one(const Camera& cam, const RenderParams& rp, const WaveBuffers& wb, uint32_t i, PixelXY p,
                        uint32_t s) {
+    const uint32_t pix = p.y * rp.width + p.x;
     Rng rng{pix, s, rp.seed};
     const CameraUs cu = camera_us(rp.strat, false, rng, cam.lens_radius > 0.0f);
-    float fx = (float)(pix % rp.width) + cu.fx, fy = (float)(pix / rp.width) + cu.fy;
+    float fx = (float)p.x + cu.fx, fy = (float)p.y + cu.fy;
     Ray r = camera_ray(cam, fx, fy, cu.time, cu.lx, cu.ly);
     wb.ray_o[i] = make_float4(r.o.x, r.o.y, r.o.z, r.t_max);
     wb.ray_d[i] = make_float4(r.d.x, r.d.y, r.d.z, r.time);
@@ -96,10 +103,11 @@ BG_D void generate_paths(const Camera& cam, const RenderParams& rp, const WaveBu
         wb.counters[C_Q0] = nitems;
         wb.counters[C_EXT_HEAD] = 0;
     }
+    // item0 split once: below, sample and pixel come from a 32-bit division
+    const uint32_t s0 = first_sample + (uint32_t)(item0 / npix), p0 = (uint32_t)(item0 % npix);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
-        uint64_t item = item0 + i;
-        generate_one(cam, rp, wb, i, pixel_of((uint32_t)(item % npix), rp.width, rp.height, rp.pixel_tiles),
-                     first_sample + (uint32_t)(item / npix));
+        const uint32_t t = p0 + i, k = t / (uint32_t)npix;
+        generate_one(cam, rp, wb, i, pixel_xy_of(t - k * (uint32_t)npix, rp.width, rp.height, rp.pixel_tiles), s0 + k);
     }
 }
 
@@ -286,7 +294,7 @@ struct VertexOut {
 // 1D k1 + 1; without, the BSDF's 2D k2 and the roulette's 1D k1), -1 where the call falls through to
 // the counter RNG.  A shade thread computes them when it picks up a path, where few registers are
 // live, into its column of shared memory (8 rows, stride SU_STRIDE).
-constexpr uint32_t SU_STRIDE = SHADE_BLOCK;
+constexpr uint32_t SU_STRIDE = SHADE_BLOCK_MAX;
 // Not inlined: renders with the independent sampler never call it, and its code (permutations, cycle
 // walking) would otherwise sit among the shade kernels' hot instructions.
 static __device__ __noinline__ void strat_prefetch(const StratParams& sp, uint32_t pix, uint32_t sample, uint64_t seed, uint32_t k1,
@@ -517,7 +525,7 @@ BG_D void finish_vertex(const WaveBuffers& wb, const GuideWave& gw, uint32_t bou
     }
 }
 
-// What a block's unit of SHADE_BLOCK paths leaves for the block-wide tail.
+// What a block's unit of paths leaves for the block-wide tail.
 struct ShadeOut {
     uint32_t slot = 0, emit_n = 0;
     bool cont = false, lrec_emit = false;
@@ -596,7 +604,7 @@ BG_D void shade_path(const Scene& sc0, const RenderParams& rp0, const WaveBuffer
     }
 }
 
-// A block's unit: entries base .. base + SHADE_BLOCK - 1 of class CLS's queue of n.
+// A block's unit: entries base .. base + blockDim.x - 1 of class CLS's queue of n.
 template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
 BG_D void shade_unit(const Scene& sc0, const RenderParams& rp0, const WaveBuffers& wb, const GuideWave& gw,
                      uint32_t bounce, uint32_t* err, const SceneRender* tab, uint32_t base, uint32_t n, float* strat_col,
@@ -608,14 +616,15 @@ BG_D void shade_unit(const Scene& sc0, const RenderParams& rp0, const WaveBuffer
                   GWK && (gw.flags & GW_RECORD) != 0, err, out.lrec_emit, append);
 }
 
-// Shades a bounce's paths of material class CLS.  One block of 512 threads per SM: 128 registers.
+// Shades a bounce's paths of material class CLS, one block per SM.
 template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
-__global__ void __launch_bounds__(SHADE_BLOCK, 1) k_shade(Scene sc0, RenderParams rp0, WaveBuffers wb, GuideWave gw,
-                                                          uint32_t bounce, uint32_t* err, const SceneRender* tab) {
+__global__ void __launch_bounds__(shade_block(GWK, TEX, INF), 1)
+    k_shade(Scene sc0, RenderParams rp0, WaveBuffers wb, GuideWave gw, uint32_t bounce, uint32_t* err, const SceneRender* tab) {
+    constexpr uint32_t BLOCK = shade_block(GWK, TEX, INF);
     __shared__ float strat_su[CLS != CLS_MISS ? 8 * SU_STRIDE : SU_STRIDE];
     __shared__ BlockAppend<3> append;
     const uint32_t n = wb.counters[C_CLS + CLS];
-    for (uint32_t base = blockIdx.x * SHADE_BLOCK; base < n; base += gridDim.x * SHADE_BLOCK) {
+    for (uint32_t base = blockIdx.x * BLOCK; base < n; base += gridDim.x * BLOCK) {
         __syncthreads();
         shade_unit<CLS, MULTI, GWK, TEX, INF, SHL>(sc0, rp0, wb, gw, bounce, err, tab, base, n, strat_su + threadIdx.x,
                                                    append);
@@ -669,7 +678,7 @@ inline int shade_launch(const Scene& sc, const RenderParams& rp, const WaveBuffe
     int n = 1;
 #define BG_CLASS(C, T, I, S)                                                                                        \
     if ((mask >> C) & 1u) {                                                                                         \
-        k_shade<C, MULTI, GWK, T, I, S><<<blocks, SHADE_BLOCK, 0, st[C]>>>(sc, rp, wb, gw, b, err, tab);             \
+        k_shade<C, MULTI, GWK, T, I, S><<<blocks, shade_block(GWK, T, I), 0, st[C]>>>(sc, rp, wb, gw, b, err, tab);             \
         ++n;                                                                                                        \
     }
     BG_CLASS(0, TEX, INF, SHL)
@@ -677,7 +686,8 @@ inline int shade_launch(const Scene& sc, const RenderParams& rp, const WaveBuffe
     BG_CLASS(2, false, INF, SHL)
     BG_CLASS(3, false, false, false)
 #undef BG_CLASS
-    k_shade<CLS_MISS, MULTI, GWK, false, false, false><<<blocks, SHADE_BLOCK, 0, st[4]>>>(sc, rp, wb, gw, b, err, tab);
+    k_shade<CLS_MISS, MULTI, GWK, false, false, false>
+        <<<blocks, shade_block(GWK, false, false), 0, st[4]>>>(sc, rp, wb, gw, b, err, tab);
     shade_join(s, fork, cs);
     return n;
 }

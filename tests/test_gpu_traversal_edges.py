@@ -100,3 +100,16 @@ def test_flat_boxes_and_axis_rays(gpu_ctx, scale):
         assert np.allclose(got["t"][hit], (want * scale)[hit], rtol=1e-5)
         assert np.array_equal(got["prim"][hit] // 2, np.where(up, first - 1, 39)[hit])
         assert np.array_equal(sc.trace(rays, any_hit=True) != 0, hit)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 4863, 4864, 4865, 9729, 155647, 155649])
+def test_short_ray_queues(gpu_ctx, n):
+    """Ray counts around one ray per warp of the persistent grid, two, and full warps: every ray gets the
+    hit it gets in a long queue (the same walk, so the same bits)."""
+    sd, rays = S.ray_soup(3000, 160_000)
+    for bvh in (A.BG_BVH_WIDE, A.BG_BVH_WIDE2):
+        sc = G.Scene(gpu_ctx, sd, bvh)
+        full, occ = sc.trace(rays), sc.trace(rays, any_hit=True)
+        got = sc.trace(rays[:n])
+        assert np.array_equal(got["prim"], full["prim"][:n]) and np.array_equal(got["t"], full["t"][:n])
+        assert np.array_equal(sc.trace(rays[:n], any_hit=True), occ[:n])
