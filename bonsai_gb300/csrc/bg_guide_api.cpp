@@ -34,6 +34,7 @@ struct bg_guide {
     float* grad = nullptr;
     float* partial = nullptr;   // per-CTA gradient slices of one batch (kept zero in unused rows)
     uint32_t partial_blocks = 0;
+    float2* loss = nullptr;     // per CTA of a batch: loss, samples with weight
     uint8_t* wpack = nullptr;
     uint32_t* step = nullptr;   // Adam step counter
     uint32_t* ctr = nullptr;    // [0] positive-weight records, [1] pool appends
@@ -217,6 +218,10 @@ bg::PoolOrder pool_order(uint32_t n, uint64_t epoch) {
     return o;
 }
 
+bg::GuideAdamState adam_state(bg_guide* g) {
+    return {g->params, g->m, g->v, g->wpack, {g->o.learning_rate, g->o.beta1, g->o.beta2, g->o.eps}};
+}
+
 // `epochs` passes over n samples in shuffled batches -> Adam steps (all asynchronous).  Returns the
 // number of steps.
 int train_batches(bg_guide* g, const float4* samples, uint32_t n, uint32_t epochs, uint64_t* epoch_counter) {
@@ -224,7 +229,7 @@ int train_batches(bg_guide* g, const float4* samples, uint32_t n, uint32_t epoch
     const uint32_t B = g->o.batch_size;
     const uint32_t nb = (n + B - 1) / B;
     cudaMemsetAsync(g->stats, 0, 2 * sizeof(float), ctx->stream);
-    bg::GuideAdam h{g->o.learning_rate, g->o.beta1, g->o.beta2, g->o.eps};
+    const bg::GuideAdamState adam = adam_state(g);
     for (uint32_t e = 0; e < epochs; ++e) {
         bg::PoolOrder order = pool_order(n, (*epoch_counter)++);
         bg::launch_guide_wsum(samples, order, B, g->wsum, ctx->stream);
@@ -238,12 +243,12 @@ int train_batches(bg_guide* g, const float4* samples, uint32_t n, uint32_t epoch
             a.wsum = g->wsum + 2 * b;
             a.alpha = g->o.alpha;
             a.partial = g->partial;
+            a.loss = g->loss;
             a.grad = g->grad;
             a.stats = g->stats;
             a.step = g->step;
             a.err = ctx->d_err;
-            bg::launch_guide_train(a, ctx->stream);
-            bg::launch_guide_adam(g->params, g->m, g->v, g->grad, g->wpack, g->step, h, ctx->stream);
+            bg::launch_guide_train(a, &adam, ctx->stream);
         }
     }
     return (int)(nb * epochs);
@@ -311,6 +316,8 @@ bg_status bg_guide_create(bg_ctx* ctx, const bg_guide_opts* opts, bg_guide** out
     if ((st = dalloc(ctx, (size_t)g->partial_blocks * bg::GUIDE_PARAMS * sizeof(float), &p, &g->allocs)) != BG_OK)
         return bail(st);
     g->partial = (float*)p;
+    if ((st = dalloc(ctx, (size_t)g->partial_blocks * sizeof(float2), &p, &g->allocs)) != BG_OK) return bail(st);
+    g->loss = (float2*)p;
     if (cudaMemsetAsync(g->partial, 0, (size_t)g->partial_blocks * bg::GUIDE_PARAMS * sizeof(float), ctx->stream) !=
         cudaSuccess)
         return bail(BG_ERR_CUDA);
@@ -368,20 +375,13 @@ bg_status bg_guide_forward(bg_guide* g, const float* queries, size_t n, float* o
     if (n == 0) return BG_OK;
     if (n >= (1u << 28)) return fail(ctx, BG_ERR_INVALID, "too many queries");
     CK(cudaSetDevice(ctx->device));
-    std::vector<float4> q(3 * n);
-    for (size_t i = 0; i < n; ++i) {
-        const float* s = queries + 9 * i;
-        q[3 * i] = make_float4(s[0], s[1], s[2], s[3]);
-        q[3 * i + 1] = make_float4(s[4], s[5], s[6], s[7]);
-        q[3 * i + 2] = make_float4(s[8], 0.0f, 0.0f, 0.0f);
-    }
+    // the caller's arrays go to the device and come back as they are: no packing on the host
     std::vector<void*> tmp;
     void *dq = nullptr, *dr = nullptr;
-    bg_status st = dalloc(ctx, q.size() * sizeof(float4), &dq, &tmp);
-    if (st == BG_OK) st = dalloc(ctx, n * bg::GUIDE_RAW_STRIDE * sizeof(float), &dr, &tmp);
-    std::vector<float> raw;
+    bg_status st = dalloc(ctx, n * BG_GUIDE_QUERY_FLOATS * sizeof(float), &dq, &tmp);
+    if (st == BG_OK) st = dalloc(ctx, n * bg::GUIDE_OUT * sizeof(float), &dr, &tmp);
     if (st == BG_OK) {
-        cudaMemcpyAsync(dq, q.data(), q.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream);
+        cudaMemcpyAsync(dq, queries, n * BG_GUIDE_QUERY_FLOATS * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
         bg::launch_guide_infer(g->wpack, (const float4*)dq, nullptr, 1, (uint32_t)n, (float*)dr, false, ctx->d_err,
                                ctx->shape.sms, ctx->stream);
         cudaError_t e = cudaGetLastError();
@@ -389,16 +389,13 @@ bg_status bg_guide_forward(bg_guide* g, const float* queries, size_t n, float* o
     }
     if (st == BG_OK) st = guide_error(ctx);
     if (st == BG_OK) {
-        raw.resize(n * bg::GUIDE_RAW_STRIDE);
-        cudaError_t e = cudaMemcpyAsync(raw.data(), dr, raw.size() * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
+        cudaError_t e = cudaMemcpyAsync(out, dr, n * bg::GUIDE_OUT * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "cudaMemcpyAsync");
     }
     cudaStreamSynchronize(ctx->stream);
     dfree_all(ctx, tmp);
-    if (st != BG_OK) return st;
-    for (size_t i = 0; i < n; ++i) std::memcpy(out + bg::GUIDE_OUT * i, raw.data() + bg::GUIDE_RAW_STRIDE * i, bg::GUIDE_OUT * sizeof(float));
-    return BG_OK;
+    return st;
 }
 
 bg_status bg_guide_gradient(bg_guide* g, const float* samples, size_t n, float* grad, float* loss) {
@@ -426,11 +423,12 @@ bg_status bg_guide_gradient(bg_guide* g, const float* samples, size_t n, float* 
             a.wsum = g->wsum;
             a.alpha = g->o.alpha;
             a.partial = g->partial;
+            a.loss = g->loss;
             a.grad = g->grad;
             a.stats = g->stats;
             a.step = nullptr;
             a.err = ctx->d_err;
-            bg::launch_guide_train(a, ctx->stream);
+            bg::launch_guide_train(a, nullptr, ctx->stream);
         }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "k_guide_train");
@@ -517,7 +515,7 @@ bg_status bg_guide_time(bg_guide* g, const float* samples, size_t n, const float
         cudaMemcpyAsync(dq, q.data(), q.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream);
         const uint32_t nb = (uint32_t)std::min<size_t>(n, g->o.batch_size);
         const bg::PoolOrder order{nb, 1u, 0u, 0u};
-        bg::GuideAdam h{g->o.learning_rate, g->o.beta1, g->o.beta2, g->o.eps};
+        const bg::GuideAdamState adam = adam_state(g);
         bg::launch_guide_wsum(ds, order, nb, g->wsum, ctx->stream);
         auto step = [&]() {
             bg::GuideTrainArgs a{};
@@ -529,12 +527,12 @@ bg_status bg_guide_time(bg_guide* g, const float* samples, size_t n, const float
             a.wsum = g->wsum;
             a.alpha = g->o.alpha;
             a.partial = g->partial;
+            a.loss = g->loss;
             a.grad = g->grad;
             a.stats = g->stats;
             a.step = g->step;
             a.err = ctx->d_err;
-            bg::launch_guide_train(a, ctx->stream);
-            bg::launch_guide_adam(g->params, g->m, g->v, g->grad, g->wpack, g->step, h, ctx->stream);
+            bg::launch_guide_train(a, &adam, ctx->stream);
         };
         auto infer = [&]() {
             bg::launch_guide_infer(g->wpack, (const float4*)dq, nullptr, 1, (uint32_t)nq, (float*)dout, true, ctx->d_err,

@@ -34,6 +34,7 @@ struct GuideTrainArgs {
     float* partial;          // per-CTA gradient slices (>= ceil(n / 128) * GUIDE_PARAMS floats; entries
                              // of unused rows stay as they are: keep them zero)
     float* grad;             // FP32 gradient accumulator (GUIDE_PARAMS): += the sum of the slices
+    float2* loss;            // per CTA: its samples' loss and how many have a weight (>= ceil(n / 128))
     float* stats;            // [0] += loss, [1] += samples with weight > 0
     uint32_t* step;          // Adam step counter, incremented once per launch (null: gradient only)
     uint32_t* err;           // error word
@@ -42,20 +43,24 @@ struct GuideTrainArgs {
 struct GuideAdam {
     float lr, beta1, beta2, eps;
 };
+struct GuideAdamState {
+    float *p, *m, *v;  // FP32 weights and moments
+    uint8_t* wpack;    // their BF16 image, rewritten
+    GuideAdam h;
+};
 
 // Forward pass over nranges (<= GUIDE_MAX_RANGES) ranges of queries: range r holds
 // min(counts[r], stride) queries from index r * stride (counts: device, null = `stride` queries in
-// every range).  out, at the same indices: raw outputs (GUIDE_RAW_STRIDE floats per query) or,
-// with mixture, the parsed mixture records of both heads, head-major (head h's record of query q
+// every range).  out, at the same indices: raw outputs (GUIDE_OUT floats per query, the queries then 9
+// floats each) or, with mixture (queries of 3 float4), the parsed mixture records of both heads, head-major (head h's record of query q
 // at (h * nranges * stride + q) * GUIDE_MIX_HEAD; out must be 16-byte aligned).
 constexpr int GUIDE_MAX_RANGES = 3;
 void launch_guide_infer(const uint8_t* wpack, const float4* query, const uint32_t* counts, uint32_t nranges,
                         uint32_t stride, float* out, bool mixture, uint32_t* err, int sms, cudaStream_t s);
 // Forward + backward of a.n samples (one CTA per 128) and the reduction of their partial
-// gradients into a.grad (two launches).
-void launch_guide_train(const GuideTrainArgs& a, cudaStream_t s);
-void launch_guide_adam(float* p, float* m, float* v, float* g, uint8_t* wpack, const uint32_t* step,
-                       const GuideAdam& h, cudaStream_t s);
+// gradients into a.grad; with `adam`, an Adam step on the accumulated gradient, which is cleared
+// (two launches).
+void launch_guide_train(const GuideTrainArgs& a, const GuideAdamState* adam, cudaStream_t s);
 void launch_guide_pack(const float* p, uint8_t* wpack, cudaStream_t s);
 // wsum[2b], wsum[2b + 1] = sums of the positive finite indirect (head 0) and direct (head 1)
 // weights of batch b (positions b*batch .. in `order`).

@@ -34,7 +34,6 @@ constexpr int GUIDE_IN_USED = 78;
 constexpr int GUIDE_PARAMS = 4 * GUIDE_HID * GUIDE_K + GUIDE_OUT_ROWS * GUIDE_K;  // 28,160
 constexpr uint32_t GUIDE_ROWGROUP_BYTES = 8 * GUIDE_K * 2;                      // 1280
 constexpr uint32_t GUIDE_WPACK_BYTES = (4 * GUIDE_HID + GUIDE_OUT_ROWS) * GUIDE_K * 2;  // 56,320
-constexpr int GUIDE_RAW_STRIDE = 96;  // floats per query in the raw output buffer
 // Mixture record of one head as the render-side inference stores it (floats): lobe i at 4i =
 // kappa * mean direction (xyz) and log(weight) + log(normalisation) - kappa, so that the density is
 // sum_i exp(m[4i+3] + m[4i..4i+2] . w); 32 + i (i < 7) = running sum of the lobe weights; 39 = c.
