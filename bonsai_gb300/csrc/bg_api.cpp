@@ -374,10 +374,12 @@ bg_status ensure_tree_wave(bg_ctx* ctx, uint32_t samples, uint32_t sh_cap, bool 
     return BG_OK;
 }
 
-bg_status check_device_error(bg_ctx* ctx, uint32_t* word) {
-    uint32_t e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+bg_status queue_error_word(bg_ctx* ctx) {
+    CK(cudaMemcpyAsync(&ctx->readback->err, ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    return BG_OK;
+}
+bg_status judge_error_word(bg_ctx* ctx, uint32_t* word) {
+    const uint32_t e = ctx->readback->err;
     if (word) *word = e;
     if (e) {
         CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
@@ -389,6 +391,12 @@ bg_status check_device_error(bg_ctx* ctx, uint32_t* word) {
         return fail(ctx, BG_ERR_DEVICE, "device error word " + std::to_string(e) + ": " + what);
     }
     return BG_OK;
+}
+bg_status check_device_error(bg_ctx* ctx, uint32_t* word) {
+    bg_status st = queue_error_word(ctx);
+    if (st != BG_OK) return st;
+    CK(cudaStreamSynchronize(ctx->stream));
+    return judge_error_word(ctx, word);
 }
 
 // Inverse of an affine 3x4 transform through the 4x4 Gauss-Jordan inverse (mat4.rs:72-140), as
@@ -524,6 +532,9 @@ bg_status bg_create(const bg_device_opts* opts, bg_ctx** out) {
     for (auto& ev : ctx->stage_ev)
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return bail(e);
     void* p;
+    if ((e = cudaMallocHost(&p, sizeof(bg_ctx::Readback))) != cudaSuccess) return bail(e);
+    ctx->readback = (bg_ctx::Readback*)p;
+    std::memset(p, 0, sizeof(bg_ctx::Readback));
     if (dalloc(ctx, 64, &p, &ctx->user) != BG_OK) return bail(cudaErrorMemoryAllocation);
     ctx->d_err = (uint32_t*)p;
     ctx->d_counters = (unsigned long long*)((char*)p + 16);
@@ -549,6 +560,7 @@ void bg_destroy(bg_ctx* ctx) {
     dfree_all(ctx, ctx->tree_allocs);
     dfree_all(ctx, ctx->film_allocs);
     dfree_all(ctx, ctx->user);
+    if (ctx->readback) cudaFreeHost(ctx->readback);
     if (ctx->flush) cudaFree(ctx->flush);
     if (ctx->ev_begin) cudaEventDestroy(ctx->ev_begin);
     if (ctx->ev_end) cudaEventDestroy(ctx->ev_end);
@@ -1324,19 +1336,29 @@ bg_status bg_trace_any_device(bg_ctx* ctx, const bg_scene* s, const bg_ray* d_ra
 static bg_status trace_host(bg_ctx* ctx, const bg_scene* s, const bg_ray* rays, size_t n, void* out, bool any) {
     if (!ctx || !s || (n && (!rays || !out))) return BG_ERR_INVALID;
     if (n == 0) return BG_OK;
+    if (!s->committed || s->ctx != ctx) return fail(ctx, BG_ERR_INVALID, "scene not committed on this context");
+    if (n >= (1ull << 31)) return fail(ctx, BG_ERR_INVALID, "too many rays");
     CK(cudaSetDevice(ctx->device));
     void *dr = nullptr, *dh = nullptr;
     std::vector<void*> tmp;
-    bg_status st = dalloc(ctx, n * sizeof(bg_ray), &dr, &tmp);
-    if (st == BG_OK) st = dalloc(ctx, n * (any ? 1 : sizeof(bg_hit)), &dh, &tmp);
+    // the hits follow the rays in one allocation
+    const size_t ray_bytes = n * sizeof(bg_ray), out_bytes = n * (any ? 1 : sizeof(bg_hit));
+    bg_status st = dalloc(ctx, ray_bytes + out_bytes, &dr, &tmp);
     if (st == BG_OK) {
-        cudaError_t e = cudaMemcpyAsync(dr, rays, n * sizeof(bg_ray), cudaMemcpyHostToDevice, ctx->stream);
+        dh = (char*)dr + ray_bytes;
+        cudaError_t e = cudaMemcpyAsync(dr, rays, ray_bytes, cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "cudaMemcpyAsync");
     }
-    if (st == BG_OK) st = trace_device(ctx, s, (const bg_ray*)dr, n, any ? nullptr : (bg_hit*)dh,
-                                       any ? (uint8_t*)dh : nullptr, any, nullptr);
     if (st == BG_OK) {
-        cudaError_t e = cudaMemcpyAsync(out, dh, n * (any ? 1 : sizeof(bg_hit)), cudaMemcpyDeviceToHost, ctx->stream);
+        const bool ref_layout = s->kind == BG_BVH_REFERENCE || s->kind == BG_BVH_REFERENCE_FIXED;
+        bg::launch_trace(s->dev, ref_layout, any, (const bg_ray*)dr, n, any ? nullptr : (bg_hit*)dh,
+                         any ? (uint8_t*)dh : nullptr, ctx->d_err, nullptr, ctx->d_head, ctx->shape, ctx->stream);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = cuda_fail(ctx, e, "k_trace");
+    }
+    if (st == BG_OK) st = check_device_error(ctx, nullptr);
+    if (st == BG_OK) {
+        cudaError_t e = cudaMemcpyAsync(out, dh, out_bytes, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "cudaMemcpyAsync");
     }
@@ -1393,6 +1415,19 @@ bg_status bgi::validate_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* 
     return BG_OK;
 }
 }  // extern "C++"
+
+// The error word, the film's NaN count and the ray counts of a render, read with one synchronisation.
+static bg_status read_render_stats(bg_ctx* ctx, const unsigned long long* ray_stats, bool rays) {
+    bg_status st = queue_error_word(ctx);
+    if (st != BG_OK) return st;
+    CK(cudaMemcpyAsync(&ctx->readback->nan, ctx->film.nan_count, sizeof(ctx->readback->nan), cudaMemcpyDeviceToHost,
+                       ctx->stream));
+    if (rays)
+        CK(cudaMemcpyAsync(ctx->readback->rays, ray_stats, sizeof(ctx->readback->rays), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return BG_OK;
+}
 
 bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const bg_render_opts* o, float* rgb_out,
                     bg_render_stats* stats) {
@@ -1540,7 +1575,9 @@ bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const 
     CK(cudaEventRecord(ctx->ev_end, ctx->stream));
     l2_window(ctx, s, false);
     uint32_t word = 0;
-    st = check_device_error(ctx, &word);
+    const bool count_rays = wavefront || (tree && ctx->tree.ray_stats);
+    if ((st = read_render_stats(ctx, wavefront ? ctx->wave.ray_stats : ctx->tree.ray_stats, count_rays)) != BG_OK) return st;
+    st = judge_error_word(ctx, &word);
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
         float ms = 0.0f;
@@ -1549,14 +1586,10 @@ bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const 
         stats->samples = total;
         stats->launches = launches;
         stats->error_word = word;
-        unsigned long long nan = 0;
-        cudaMemcpy(&nan, ctx->film.nan_count, sizeof(nan), cudaMemcpyDeviceToHost);
-        stats->nan_samples = nan;
-        if (wavefront || (tree && ctx->tree.ray_stats)) {
-            unsigned long long rs[2] = {0, 0};
-            cudaMemcpy(rs, wavefront ? ctx->wave.ray_stats : ctx->tree.ray_stats, sizeof(rs), cudaMemcpyDeviceToHost);
-            stats->extension_rays = rs[0];
-            stats->shadow_rays = rs[1];
+        stats->nan_samples = ctx->readback->nan;
+        if (count_rays) {
+            stats->extension_rays = ctx->readback->rays[0];
+            stats->shadow_rays = ctx->readback->rays[1];
         }
         if (timing) {
             double ext = 0, shade = 0, shadow = 0;
@@ -1721,7 +1754,8 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
     }
     CK(cudaEventRecord(ctx->ev_end, ctx->stream));
     uint32_t word = 0;
-    st = check_device_error(ctx, &word);
+    st = read_render_stats(ctx, ctx->wave.ray_stats, true);
+    if (st == BG_OK) st = judge_error_word(ctx, &word);
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
         float ms = 0.0f;
@@ -1730,12 +1764,9 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
         stats->samples = total_items;
         stats->launches = launches;
         stats->error_word = word;
-        unsigned long long nan = 0, rs[2] = {0, 0};
-        cudaMemcpy(&nan, ctx->film.nan_count, sizeof(nan), cudaMemcpyDeviceToHost);
-        cudaMemcpy(rs, ctx->wave.ray_stats, sizeof(rs), cudaMemcpyDeviceToHost);
-        stats->nan_samples = nan;
-        stats->extension_rays = rs[0];
-        stats->shadow_rays = rs[1];
+        stats->nan_samples = ctx->readback->nan;
+        stats->extension_rays = ctx->readback->rays[0];
+        stats->shadow_rays = ctx->readback->rays[1];
     }
     if (st == BG_OK) {
         pix0 = 0;

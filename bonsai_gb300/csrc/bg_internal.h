@@ -20,6 +20,13 @@ struct bg_ctx {
     bg::LaunchShape shape{1, 128};
     uint32_t max_queue = 1u << 22;
     uint32_t* d_err = nullptr;
+    // what a call reads back about its launches, page-locked so that the copies queue up behind the
+    // kernels and one synchronisation covers them
+    struct Readback {
+        uint32_t err;
+        uint32_t pad;
+        unsigned long long nan, rays[2];
+    }* readback = nullptr;
     unsigned long long* d_counters = nullptr;
     uint32_t* d_head = nullptr;
     bg::FilmBuffers film{};
@@ -105,6 +112,9 @@ bg::Camera make_camera(const bg_camera& c);
 bg_status ensure_film(bg_ctx* ctx, uint32_t w, uint32_t h);
 bg_status ensure_wave(bg_ctx* ctx, uint32_t cap);
 bg_status check_device_error(bg_ctx* ctx, uint32_t* word);
+// Its two halves: queue the read-back of the error word; after a synchronisation, look at it.
+bg_status queue_error_word(bg_ctx* ctx);
+bg_status judge_error_word(bg_ctx* ctx, uint32_t* word);
 // Scene bounds padded slightly: p_norm = (p - lo) * inv lies in [0, 1) for every primitive.
 void scene_bounds(const bg_scene* s, float lo[3], float inv[3]);
 // Shared argument checks of bg_render / bg_render_guided.
