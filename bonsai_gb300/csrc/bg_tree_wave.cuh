@@ -126,9 +126,17 @@ __global__ void __launch_bounds__(TW_SHADE_BLOCK, 1) k_tw_shade(Scene sc, Render
     const bool deeper = d + 1 < rp.max_depth;
     const uint32_t stride = gridDim.x * blockDim.x;
     __shared__ BlockAppend<2> append;
+    __shared__ BlockGroup<6> group;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         __syncthreads();
-        const uint32_t i = base + threadIdx.x;
+        // the block's nodes grouped by material class: a warp of glass skips the lights, one of matte
+        // the children, and neither walks the other's BSDF code
+        uint32_t key = 5;
+        if (base + threadIdx.x < n) {
+            const int hp = tw.hit[base + threadIdx.x].x;
+            key = hp < 0 ? 4u : (uint32_t)sc.prim_cls[hp];
+        }
+        const uint32_t i = base + group(key);
         bool valid = i < n;
         uint4 meta = make_uint4(0, 1, 0, 0);
         RGB beta = rgb(0.0f);
@@ -169,13 +177,15 @@ __global__ void __launch_bounds__(TW_SHADE_BLOCK, 1) k_tw_shade(Scene sc, Render
             bsdf = make_bsdf<-1, false>(sc, it, have_tp ? &tp : nullptr, false);
             add_L(tw, slot, beta * emitted_radiance(sc, it, it.wo));
         }
-        // light sampling: loops with the same trip count on every lane (warp-collective appends)
+        // specular BSDFs have no value for a light's direction
+        const bool lit = valid && bsdf.num_components(BSDF_ALL & ~BSDF_SPECULAR) > 0;
+        // light sampling: loops with the same trip count on every thread (block-collective appends)
         if (sc.nlights > 0) {
             if constexpr (KIND == 1) {  // whitted.rs:176-192
                 for (uint32_t j = 0; j < sc.nlights; ++j) {
                     __syncthreads();
                     TwShadow sh[2];
-                    if (valid) {
+                    if (lit) {
                         LightSample ls = light_sample_any<false>(sc, sc.light_prims[j], it, rng.u(TW_DIM_LIGHTS + 2 * j),
                                                              rng.u(TW_DIM_LIGHTS + 2 * j + 1));
                         if (!is_black(ls.radiance) && ls.pdf != 0.0f) {
@@ -194,7 +204,7 @@ __global__ void __launch_bounds__(TW_SHADE_BLOCK, 1) k_tw_shade(Scene sc, Render
                     __syncthreads();
                     float u[4];
                     rng.block(TW_DIM_LIGHTS + 4 * j, u);
-                    direct_rays(sc, tw, valid, it, bsdf, sc.light_prims[j], u[2], u[3], u[0], u[1], beta / 1.0f, slot,
+                    direct_rays(sc, tw, lit, it, bsdf, sc.light_prims[j], u[2], u[3], u[0], u[1], beta / 1.0f, slot,
                                 append);
                 }
             } else {  // uniform_sample_one_light (integrator.rs:309-328)
@@ -203,7 +213,7 @@ __global__ void __launch_bounds__(TW_SHADE_BLOCK, 1) k_tw_shade(Scene sc, Render
                 rng.block(TW_DIM_LIGHTS + 4, u + 4);
                 const float count = (float)sc.nlights;
                 const uint32_t li = (uint32_t)rmin(u[0] * count, count - 1.0f);
-                direct_rays(sc, tw, valid, it, bsdf, sc.light_prims[li], u[3], u[4], u[1], u[2], beta / (1.0f / count),
+                direct_rays(sc, tw, lit, it, bsdf, sc.light_prims[li], u[3], u[4], u[1], u[2], beta / (1.0f / count),
                             slot, append);
             }
         }

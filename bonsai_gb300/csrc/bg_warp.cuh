@@ -64,6 +64,44 @@ struct BlockAppend {
     }
 };
 
+// A block's threads grouped by key (0 .. NK - 1): returns the thread whose item this thread takes, so
+// that warps hold one key each but for NK - 1 borders.  Every thread of the block calls it (three
+// barriers); `sm` is free again after the next barrier.
+template <int NK>
+struct BlockGroup {
+    uint32_t n[NK][32];
+    uint16_t item[1024];
+    BG_D uint32_t operator()(uint32_t key) {
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+        uint32_t own = 0;
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            const uint32_t mask = __ballot_sync(FULL, key == (uint32_t)k);
+            if (lane == 0) n[k][warp] = __popc(mask);
+            if (key == (uint32_t)k) own = __popc(mask & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        if (warp == 0) {  // exclusive sums, key by key
+            uint32_t base = 0;
+            for (int k = 0; k < NK; ++k) {
+                const uint32_t c = lane < nwarps ? n[k][lane] : 0u;
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= (uint32_t)o) incl += t;
+                }
+                if (lane < nwarps) n[k][lane] = base + incl - c;
+                base += __shfl_sync(FULL, incl, 31);
+            }
+        }
+        __syncthreads();
+        item[n[key][warp] + own] = (uint16_t)threadIdx.x;
+        __syncthreads();
+        return item[threadIdx.x];
+    }
+};
+
 BG_D Ray load_ray(float4 o, float4 d) {
     Ray r;
     r.o = f4xyz(o);
