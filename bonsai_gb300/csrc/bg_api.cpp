@@ -301,6 +301,21 @@ bg_status ensure_wave(bg_ctx* ctx, uint32_t cap) {
     return BG_OK;
 }
 
+uint32_t wave_limit(const bg_ctx* ctx) {
+    if (ctx->max_queue != kDefaultQueue) return ctx->max_queue;
+    return ctx->cap ? kFallbackQueue : ctx->queue_fit;
+}
+
+bg_status ensure_wave_for(bg_ctx* ctx, uint64_t total, uint32_t* cap) {
+    for (;;) {
+        *cap = (uint32_t)std::min<uint64_t>(wave_limit(ctx), std::max<uint64_t>(total, 1));
+        const bg_status st = ensure_wave(ctx, *cap);
+        if (st != BG_ERR_OOM || ctx->max_queue != kDefaultQueue || *cap <= kFallbackQueue) return st;
+        cudaGetLastError();  // the failed allocation's
+        ctx->queue_fit = std::max(kFallbackQueue, *cap / 2);
+    }
+}
+
 // L2 access-policy window over the scene's 8-wide traversal range (nodes + leaf primitives): its
 // lines persist in the L2 set-aside while the wave state streams past them.  The set-aside is
 // requested for the render and given back after it (limit 0, persisting lines reset), so nothing
@@ -1454,8 +1469,7 @@ bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const 
     bool wavefront = !tree && (o->mode == BG_MODE_PBRT && (s->kind == BG_BVH_WIDE || s->kind == BG_BVH_WIDE2));
     uint32_t cap = 0;
     if (wavefront) {
-        cap = (uint32_t)std::min<uint64_t>(ctx->max_queue, std::max<uint64_t>(total, 1));
-        if ((st = ensure_wave(ctx, cap)) != BG_OK) return st;
+        if ((st = ensure_wave_for(ctx, total, &cap)) != BG_OK) return st;
     }
     const bool timing = wavefront && (o->flags & BG_RENDER_STAGE_TIMING);
     const uint64_t nwaves = wavefront ? (total + cap - 1) / cap : 0;
@@ -1691,8 +1705,8 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
     }
     const bg::SceneRender* d_tab = ctx->batch_tab;
     CK(cudaMemcpyAsync(ctx->batch_tab, tab.data(), n * sizeof(bg::SceneRender), cudaMemcpyHostToDevice, ctx->stream));
-    const uint32_t cap = (uint32_t)std::min<uint64_t>(ctx->max_queue, std::max<uint64_t>(total_items, 1));
-    if ((st = ensure_wave(ctx, cap)) != BG_OK) {
+    uint32_t cap = 0;
+    if ((st = ensure_wave_for(ctx, total_items, &cap)) != BG_OK) {
         dfree_all(ctx, tmp);
         return st;
     }

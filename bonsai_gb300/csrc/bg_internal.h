@@ -11,6 +11,13 @@
 #include "../../include/bonsai_gpu.h"
 #include "bg_kernels.h"
 
+// Paths per wave unless the caller says otherwise.  Every stage of a wave ends with a few long rays on an
+// almost idle GPU (0.2 ms a bounce on the production scene), so fewer waves are better until the
+// path state (about 230 bytes a path, 7.7 GB here) is a burden: production frame at 16 spp (33M paths)
+// 93.2 ms with waves of 2^22, 85.1 / 81.0 / 79.0 with 2^23 / 2^24 / 2^25; example scene (16.8M paths) 4.85 /
+// 4.33 / 4.08 / 4.08.  Under a memory cap, and where that much is not to be had, waves of kFallbackQueue.
+constexpr uint32_t kDefaultQueue = 1u << 25, kFallbackQueue = 1u << 22;
+
 struct bg_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -18,7 +25,8 @@ struct bg_ctx {
     uint64_t cap = 0, used = 0;
     bg::ShadeFork fork{};           // streams / events of BG_TUNE_CONCURRENT_SHADE
     bg::LaunchShape shape{1, 128};
-    uint32_t max_queue = 1u << 22;
+    uint32_t max_queue = kDefaultQueue;
+    uint32_t queue_fit = kDefaultQueue;  // the largest default wave that has not failed to allocate
     uint32_t* d_err = nullptr;
     // what a call reads back about its launches, page-locked so that the copies queue up behind the
     // kernels and one synchronisation covers them
@@ -111,6 +119,10 @@ void dfree_all(bg_ctx* ctx, std::vector<void*>& v);
 bg::Camera make_camera(const bg_camera& c);
 bg_status ensure_film(bg_ctx* ctx, uint32_t w, uint32_t h);
 bg_status ensure_wave(bg_ctx* ctx, uint32_t cap);
+// Paths per wave before a render's own total bounds them; ensure_wave for `total` paths (*cap = paths
+// per wave).
+uint32_t wave_limit(const bg_ctx* ctx);
+bg_status ensure_wave_for(bg_ctx* ctx, uint64_t total, uint32_t* cap);
 bg_status check_device_error(bg_ctx* ctx, uint32_t* word);
 // Its two halves: queue the read-back of the error word; after a synchronisation, look at it.
 bg_status queue_error_word(bg_ctx* ctx);
