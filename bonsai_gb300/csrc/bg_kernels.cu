@@ -414,25 +414,40 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
         double s[3] = {0.0, 0.0, 0.0}, q[3] = {0.0, 0.0, 0.0};
         float ps[3] = {0.0f, 0.0f, 0.0f};
         uint32_t cnt = 0, nan = 0;
-        for (uint64_t j = i; j < end; j += npix) {
-            const float4 l4 = wb.L[j];
-            RGB L = apply_pending(wb, (uint32_t)j, rgb(l4.x, l4.y, l4.z), wb.state[j], nlights);
-            const float y = luminance(L);
-            if (is_nan(L) || y < -1e-5f || isinf(y)) {
-                L = rgb(0.0f);
-                ++nan;
+        // four samples' loads in flight
+        for (uint64_t j0 = i; j0 < end; j0 += 4 * npix) {
+            float4 l4[4];
+            uint32_t st[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t j = j0 + k * npix;
+                if (j < end) {
+                    l4[k] = wb.L[j];
+                    st[k] = wb.state[j];
+                }
             }
-            const double r = L.r, g = L.g, b = L.b;
-            s[0] += r;
-            s[1] += g;
-            s[2] += b;
-            q[0] += r * r;
-            q[1] += g * g;
-            q[2] += b * b;
-            ps[0] += L.r;
-            ps[1] += L.g;
-            ps[2] += L.b;
-            ++cnt;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t j = j0 + k * npix;
+                if (j >= end) break;
+                RGB L = apply_pending(wb, (uint32_t)j, rgb(l4[k].x, l4[k].y, l4[k].z), st[k], nlights);
+                const float y = luminance(L);
+                if (is_nan(L) || y < -1e-5f || isinf(y)) {
+                    L = rgb(0.0f);
+                    ++nan;
+                }
+                const double r = L.r, g = L.g, b = L.b;
+                s[0] += r;
+                s[1] += g;
+                s[2] += b;
+                q[0] += r * r;
+                q[1] += g * g;
+                q[2] += b * b;
+                ps[0] += L.r;
+                ps[1] += L.g;
+                ps[2] += L.b;
+                ++cnt;
+            }
         }
         const size_t pix = wb.pixel[i];
 #pragma unroll

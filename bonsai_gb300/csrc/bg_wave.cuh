@@ -86,7 +86,8 @@ BG_D void generate_one(const Camera& cam, const RenderParams& rp, const WaveBuff
                        uint32_t s) {
     const uint32_t pix = p.y * rp.width + p.x;
     Rng rng{pix, s, rp.seed};
-    const CameraUs cu = camera_us(rp.strat, false, rng, cam.lens_radius > 0.0f);
+    // without the time sample: nothing in a scene moves, so no path depends on its ray's time
+    const CameraUs cu = camera_us(rp.strat, false, rng, cam.lens_radius > 0.0f, false);
     float fx = (float)p.x + cu.fx, fy = (float)p.y + cu.fy;
     Ray r = camera_ray(cam, fx, fy, cu.time, cu.lx, cu.ly);
     wb.ray_o[i] = make_float4(r.o.x, r.o.y, r.o.z, r.t_max);
