@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(BIN_BLOCK) k_bin(Scene sc0, WaveBuffers wb, ui
             Isect it;
             GuideQuery gq{make_float4(0.5f, 0.5f, 0.5f, 0.0f), make_float4(0.0f, 1.0f, 0.0f, 0.0f),
                           make_float4(1.0f, 0.0f, 0.0f, 0.0f)};
-            if (prim_isect(sc0, wb.hit[slot].x, ray, &it)) gq = make_query(gw, it, -ray.d);
+            if (prim_isect<true>(sc0, wb.hit[slot].x, ray, &it)) gq = make_query(gw, it, -ray.d);
             float4* o = gw.query + 3 * (size_t)qpos;
             o[0] = gq.a;
             o[1] = gq.b;

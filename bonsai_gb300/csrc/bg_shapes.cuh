@@ -657,9 +657,16 @@ BG_D void load_tri(const Scene& sc, uint32_t prim, V3* p0, V3* p1, V3* p2) {
     *p2 = f4xyz(c);
 }
 
+static __device__ __noinline__ bool quadric_isect_call(const float4* q, const Ray& ray, Isect* it, SurfaceGeom* g) {
+    float t;
+    return quadric_hit(q, ray, INFINITY, &t, it, g);
+}
 // Full closest-hit interaction for a primitive given the ray (re-runs the shape test with
 // t_max = infinity, which reproduces the traversal's t, barycentrics and hit side).
-// With `g`, also the surface parameterisation and partials (SurfaceGeom).
+// With `g`, also the surface parameterisation and partials (SurfaceGeom).  COLD_QUADRICS keeps the three
+// quadrics out of line (31 of a matte shade kernel's 143 KB, and its spills): Cornell box 1.715 -> 1.675 ms,
+// preview 396 -> 390 us; the textured kernels lose 3% to the call and keep them inline.
+template <bool COLD_QUADRICS = false>
 BG_D bool prim_isect(const Scene& sc, int prim, const Ray& ray, Isect* it, SurfaceGeom* g = nullptr) {
     if ((uint32_t)prim < sc.ntri) {
         V3 p0, p1, p2;
@@ -674,8 +681,18 @@ BG_D bool prim_isect(const Scene& sc, int prim, const Ray& ray, Isect* it, Surfa
         if (!sphere_test(s, ray, INFINITY, &h)) return false;
         sphere_isect(s, h, ray, it, g);
     } else {
-        float t;
-        if (!quadric_hit(sc.quads + QUADRIC_F4 * (prim - sc.ntri - sc.nsph), ray, INFINITY, &t, it, g)) return false;
+        const float4* q = sc.quads + QUADRIC_F4 * (prim - sc.ntri - sc.nsph);
+        if constexpr (COLD_QUADRICS) {
+            Isect i2;  // copies: `it` and `ray` stay in registers
+            SurfaceGeom g2;
+            const Ray r2 = ray;
+            if (!quadric_isect_call(q, r2, &i2, g ? &g2 : nullptr)) return false;
+            *it = i2;
+            if (g) *g = g2;
+        } else {
+            float t;
+            if (!quadric_hit(q, ray, INFINITY, &t, it, g)) return false;
+        }
     }
     it->prim = prim;
     return true;

@@ -298,10 +298,12 @@ struct VertexOut {
 constexpr uint32_t SU_STRIDE = SHADE_BLOCK_MAX;
 // Not inlined: renders with the independent sampler never call it, and its code (permutations, cycle
 // walking) would otherwise sit among the shade kernels' hot instructions.
+// The second 1D value is the roulette's when the bounce samples a light, and only bounces past the
+// third roll it.
 static __device__ __noinline__ void strat_prefetch(const StratParams& sp, uint32_t pix, uint32_t sample, uint64_t seed, uint32_t k1,
-                         uint32_t k2, float* col) {
+                         uint32_t k2, bool roulette, float* col) {
     col[0] = k1 < sp.dims ? strat_1d(sp, false, pix, sample, seed, k1) : -1.0f;
-    col[SU_STRIDE] = k1 + 1 < sp.dims ? strat_1d(sp, false, pix, sample, seed, k1 + 1) : -1.0f;
+    col[SU_STRIDE] = roulette && k1 + 1 < sp.dims ? strat_1d(sp, false, pix, sample, seed, k1 + 1) : -1.0f;
     for (uint32_t j = 0; j < 3; ++j) {
         const float2 v = k2 + j < sp.dims ? strat_2d(sp, false, pix, sample, seed, k2 + j) : make_float2(-1.0f, -1.0f);
         col[(2 + 2 * j) * SU_STRIDE] = v.x;
@@ -558,7 +560,8 @@ BG_D void shade_path(const Scene& sc0, const RenderParams& rp0, const WaveBuffer
     float eta_scale = b4.w;
     const float* su = nullptr;
     if (CLS != CLS_MISS && rp.strat.dims > 0) {
-        strat_prefetch(rp.strat, wb.pixel[slot], wb.sample[slot], rp.seed, st_k1(state), st_k2(state), strat_col);
+        strat_prefetch(rp.strat, wb.pixel[slot], wb.sample[slot], rp.seed, st_k1(state), st_k2(state), bounce > 3,
+                       strat_col);
         su = strat_col;
     }
     float4 l4 = bounce ? wb.L[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -568,7 +571,7 @@ BG_D void shade_path(const Scene& sc0, const RenderParams& rp0, const WaveBuffer
     state &= ~(ST_PENDING | ST_LREC);
     bool specular_bounce = (state & ST_SPECULAR) != 0;
     Isect it;
-    bool hit = CLS != CLS_MISS && prim >= 0 && prim_isect(sc, prim, ray, &it);
+    bool hit = CLS != CLS_MISS && prim >= 0 && prim_isect<!TEX>(sc, prim, ray, &it);
     const bool counted = bounce == 0 || specular_bounce;
     const bool rec_open = record && (state & ST_REC_OPEN);
     RGB le = hit && (counted || rec_open) ? emitted_radiance(sc, it, -ray.d) : rgb(0.0f);
