@@ -97,11 +97,6 @@ void launch_trace(const Scene& sc, bool ref_layout, bool any, const bg_ray* rays
 #undef BG_TRACE
 }
 
-// Chained launches (launch_chained).  A kernel's last blocks let the next kernel's start where SMs
-// become free; that kernel's blocks wait for this one's end, and for its writes, before they touch memory.
-BG_D void allow_next() { cudaTriggerProgrammaticLaunchCompletion(); }
-BG_D void wait_previous() { cudaGridDependencySynchronize(); }
-
 // Batch: item -> scene by binary search over the scenes' first items, then as above.
 __global__ void k_generate_batch(const SceneRender* tab, uint32_t nscenes, WaveBuffers wb, uint64_t item0,
                                  uint32_t nitems) {
@@ -470,26 +465,6 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
         f.count[pix] += cnt;
         if (nan) atomicAdd(f.nan_count, (unsigned long long)nan);
     }
-}
-
-// Launches a kernel that starts with wait_previous() behind the previous kernel of its stream: its
-// blocks may come to the SMs that the previous one has left while that one still ends.  Generation,
-// extension and binning, and a bounce's shadow rays and the next extension (the shade launches wait for
-// events of several streams): a 64 x 64 preview 388 -> 357 us, 256 x 256 x 16 Cornell paths 1.669 -> 1.647
-// ms; a wave of many paths gains nothing, nor does a batch, whose graph's launches are short already
-// (3.43 and 3.44 ms: launched plainly).
-template <class... P, class... Args>
-static void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 static int launch_bounces(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t* err,

@@ -27,6 +27,7 @@ namespace bg {
 
 // The wave's camera samples as the level-0 nodes (node id 1, depth 0).
 __global__ void k_tw_gen(Camera cam, RenderParams rp, TreeWave tw, uint64_t item0, uint32_t n) {
+    allow_next();
     const uint64_t npix = (uint64_t)rp.width * rp.height;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         tw.counters[0] = n;
@@ -53,14 +54,8 @@ __global__ void k_tw_gen(Camera cam, RenderParams rp, TreeWave tw, uint64_t item
     }
 }
 
-// Before level d: the next level's queue and the shadow queue start empty.
-__global__ void k_tw_prep(TreeWave tw, uint32_t d) {
-    tw.counters[(d + 1) & 1] = 0;
-    tw.counters[TW_SHADOW] = 0;
-    tw.counters[TW_EXT_HEAD] = 0;
-    tw.counters[TW_SH_HEAD] = 0;
-}
-
+// The counters are reset by kernels that precede the next use and follow the last one: the next level's
+// queue, the shadow queue and its head by extension, the extension's head by the shadow rays.
 struct TwExtSrc {
     TreeWave tw;
     uint32_t b;
@@ -74,8 +69,15 @@ struct TwExtSrc {
 template <int LAYOUT>
 __global__ void __launch_bounds__(128, BG_MINBLOCKS) k_tw_extend(Scene sc, TreeWave tw, uint32_t d, uint32_t* err,
                                                                  int refill) {
+    allow_next();
+    wait_previous();
     const uint32_t n = min(tw.counters[d & 1], tw.cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&tw.ray_stats[0], (unsigned long long)n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(&tw.ray_stats[0], (unsigned long long)n);
+        tw.counters[(d + 1) & 1] = 0;
+        tw.counters[TW_SHADOW] = 0;
+        tw.counters[TW_SH_HEAD] = 0;
+    }
     TwExtSrc src{tw, d & 1u};
 #if BG_SMEM_STACK
     __shared__ uint2 stack8[LAYOUT == 8 ? STACK8 * 128 : 1];
@@ -108,8 +110,13 @@ struct TwShadowSrc {
 
 template <int LAYOUT>
 __global__ void __launch_bounds__(128, BG_MINBLOCKS) k_tw_shadow(Scene sc, TreeWave tw, uint32_t* err, int refill) {
+    allow_next();
+    wait_previous();
     const uint32_t n = min(tw.counters[TW_SHADOW], tw.sh_cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&tw.ray_stats[1], (unsigned long long)n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(&tw.ray_stats[1], (unsigned long long)n);
+        tw.counters[TW_EXT_HEAD] = 0;
+    }
     TwShadowSrc src{tw};
 #if BG_SMEM_STACK
     __shared__ uint2 stack8[LAYOUT == 8 ? STACK8 * 128 : 1];
@@ -139,14 +146,13 @@ int launch_tree_wave(int kind, const Scene& sc, const Camera& cam, const RenderP
     const dim3 shade_grid(std::max(1u, (uint32_t)(ls.sms * ls.blocks_per_sm) * 128u / TW_SHADE_BLOCK));
     const bool wide8 = sc.nodes8 != nullptr;
     for (uint32_t d = 0; d < rp.max_depth; ++d) {
-        k_tw_prep<<<1, 1, 0, s>>>(tw, d);
-        if (wide8) k_tw_extend<8><<<grid, block, 0, s>>>(sc, tw, d, err, ls.refill);
-        else k_tw_extend<2><<<grid, block, 0, s>>>(sc, tw, d, err, ls.refill);
+        if (wide8) launch_chained(k_tw_extend<8>, grid, block, s, sc, tw, d, err, ls.refill);
+        else launch_chained(k_tw_extend<2>, grid, block, s, sc, tw, d, err, ls.refill);
         if (kind == 1) launch_tw_shade_whitted(sc, rp, tw, d, item0, err, shade_grid, s);
         else launch_tw_shade_direct(kind, sc, rp, tw, d, item0, err, shade_grid, s);
-        if (wide8) k_tw_shadow<8><<<grid, block, 0, s>>>(sc, tw, err, ls.refill);
-        else k_tw_shadow<2><<<grid, block, 0, s>>>(sc, tw, err, ls.refill);
-        launches += 4;
+        if (wide8) launch_chained(k_tw_shadow<8>, grid, block, s, sc, tw, err, ls.refill);
+        else launch_chained(k_tw_shadow<2>, grid, block, s, sc, tw, err, ls.refill);
+        launches += 3;
     }
     return launches;
 }

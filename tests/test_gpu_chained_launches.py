@@ -31,3 +31,21 @@ def test_same_film_as_separate_launches(gpu_ctx, kind, layout, w, h, spp, sort, 
             assert np.array_equal(r.rgb, apart)
     finally:
         autotune.set_(gpu_ctx, old.refill, old.blocks_per_sm, old.wave_paths)
+
+
+@pytest.mark.parametrize("integrator", ["whitted", "direct"])
+@pytest.mark.parametrize("layout", [A.BG_BVH_WIDE, A.BG_BVH_WIDE2])
+@pytest.mark.parametrize("w,h,spp,depth", [(1, 1, 1, 1), (33, 1, 1, 2), (127, 5, 2, 5), (64, 64, 1, 8)])
+def test_tree_levels_equal_the_per_thread_kernel(gpu_ctx, integrator, layout, w, h, spp, depth):
+    """The tree wavefront's levels against one thread per sample over the reference layout: the same
+    trees; the sums differ in order and contraction, so all but a few channels (hits of rays at an
+    edge, 1e-2 of them at the most) are equal to 1e-4 of their size."""
+    sd = S.cornell(w, h, spp=spp)
+    integ = {"whitted": lambda: G.WhittedIntegrator(sd.camera, spp, depth),
+             "direct": lambda: G.DirectLightingIntegrator(sd.camera, spp, depth)}[integrator]()
+    ref = integ.render(G.Scene(gpu_ctx, sd, A.BG_BVH_REFERENCE)).rgb
+    sc = G.Scene(gpu_ctx, sd, layout)
+    for _ in range(3):
+        r = integ.render(sc)
+        assert r.stats.error_word == 0
+        assert np.mean(np.abs(r.rgb - ref) <= 1e-4 * (1.0 + np.abs(ref))) >= 0.99
