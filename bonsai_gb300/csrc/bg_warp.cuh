@@ -118,7 +118,7 @@ BG_D void wait_previous() { cudaGridDependencySynchronize(); }
 
 // Launches a kernel that starts with wait_previous() behind the previous kernel of its stream: its
 // blocks may come to the SMs that the previous one has left while that one still ends.  Path waves:
-// extension and binning (the shade launches wait for events of several streams): a 64 x 64 preview
+// extension and binning (the shade launches wait for events of several streams): a 67 x 49 preview
 // 388 -> 357 us, 256 x 256 x 16 Cornell paths 1.669 -> 1.647 ms; a wave of many paths gains nothing,
 // nor does a batch, whose graph's launches are short already (3.43 and 3.44 ms: launched plainly).
 // Tree waves: extension and shadow rays, and no launch of its own for the counters' resets: 4096 Whitted
