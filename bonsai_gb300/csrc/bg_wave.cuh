@@ -638,8 +638,11 @@ __global__ void __launch_bounds__(shade_block(GWK, TEX, INF), 1)
 // Streams of one bounce's class kernels.  The classes share no data a kernel of another class
 // reads (each shades its own queue's paths, writes only those paths' slots and appends to the next
 // queues and the training pool with atomics), so with a fork they run side by side: the first class the
-// scene has on the launching stream, every other one on a fork stream, which first waits for everything
-// already on `s`, and the misses behind the last class; shade_join makes `s` wait for them again.
+// scene has on the launching stream, every other one and the misses each on a fork stream, which first
+// waits for everything already on `s`; shade_join makes `s` wait for them again.  (The misses behind
+// the last class, often the heaviest, against on their own: a 67 x 49 preview 355 and 322 us, 256 x 256 x 16
+// Cornell paths 1.647 and 1.622 ms, the textured room 3.047 and 2.990; behind the first class 325 us,
+// 1.600 and 3.052.)
 // Only the classes of `mask` (Scene::cls_mask) take launches and event calls: all five of every scene
 // were 5 launches and 13 event calls a bounce, most of a small film's time on the host.
 struct ClassStreams {
@@ -649,19 +652,16 @@ struct ClassStreams {
 inline ClassStreams shade_fork(cudaStream_t s, const ShadeFork* fork, uint32_t mask) {
     ClassStreams cs{{s, s, s, s, s}};
     if (!fork) return cs;
-    cudaStream_t last = s;
     bool first = true;
-    for (int c = 0; c < 4; ++c) {
-        if (!((mask >> c) & 1u)) continue;
+    for (int c = 0; c < 5; ++c) {
+        if (c < CLS_MISS && !((mask >> c) & 1u)) continue;
         if (!first) {
             if (cs.used == 0) cudaEventRecord(fork->fork, s);
             cudaStreamWaitEvent(fork->aux[cs.used], fork->fork, 0);
-            last = fork->aux[cs.used++];
+            cs.st[c] = fork->aux[cs.used++];
         }
         first = false;
-        cs.st[c] = last;
     }
-    cs.st[4] = last;
     return cs;
 }
 inline void shade_join(cudaStream_t s, const ShadeFork* fork, const ClassStreams& cs) {
