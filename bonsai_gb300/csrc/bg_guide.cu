@@ -7,8 +7,9 @@
 //                  activations of all layers stay in shared memory, dX = dZ W and
 //                  dW = dZ^T H run as MN-major MMAs on the same tiles, each CTA stores its weight
 //                  gradient (plain stores, no atomics) into its slice of a partial buffer.
-//   k_guide_reduce sums the CTAs' partial gradients into the FP32 gradient and, in training, takes the
-//                  Adam step on the FP32 master weights and rewrites the BF16 core-matrix image.
+//   k_guide_reduce sums the CTAs' partial gradients into the FP32 gradient (k_guide_reduce_ordered: in a
+//                  fixed order).
+//   k_guide_adam   Adam on the FP32 master weights; rewrites the BF16 core-matrix image.
 // Both network kernels bring the weight image into shared memory with one bulk (TMA) copy.
 //
 // Shared-memory tiles (no swizzle, core matrices of 8 rows x 16 B, see bg_umma.cuh):
@@ -534,16 +535,54 @@ __device__ __forceinline__ void pack_param(uint8_t* wpack, int i, float p) {
     *reinterpret_cast<__nv_bfloat16*>(wpack + guide_wpack_off(l) + core_off(r, c, ACT_RS)) = __float2bfloat16_rn(p);
 }
 
+// The batch's loss from its CTAs' (one warp).
+BG_D void add_losses(const GuideTrainArgs& a, uint32_t n, uint32_t lane) {
+    double l = 0.0, c = 0.0;
+    for (uint32_t k = lane; k < n; k += 32) {
+        l += a.loss[k].x;
+        c += a.loss[k].y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (lane == 0) {
+        a.stats[0] += (float)l;
+        a.stats[1] += (float)c;
+    }
+}
+
 // grad[i] += sum over the n CTAs' partial gradients (parameter i of slice b at b * GUIDE_PARAMS + i), and
 // the CTAs' losses into stats.  REDUCE_SPLIT threads share a parameter, each taking every
-// REDUCE_SPLIT-th slice with two sums in flight; their sums are added in a fixed order, so a batch gives
-// the same bits every time (FP32 atomics in any order before).  ADAM: the Adam step of the parameter
-// follows at once, with `grad` and the optimiser state read and written once: 17 steps of 16,384 samples
-// took 92 us of reductions and 93 us of Adam kernels of their own.
+// REDUCE_SPLIT-th slice with two sums in flight (more loads in flight than one thread walking all
+// slices; bound by those loads' latency: 14 MB of slices a batch of 16,384, mostly from L2).
+//
+// The two kernels differ in how those threads' sums meet.  k_guide_reduce, in training, adds them as
+// they arrive.  One order is as good as another for a sum, but the weights of an epoch depend on it: a last
+// bit of a gradient turns a BF16 rounding of a weight, that the next step's activations, and Adam's
+// division by sqrt(v) makes whole learning-rate steps of a change in a gradient near zero.  So an
+// epoch of 16 steps with the sums in a fixed order is up to 1e-3 (relative) from one with the sums as they
+// arrive, as two of the latter may be from each other; a program's weights stay as they are only while
+// the launches that sum them do.  k_guide_reduce_ordered, for the gradient by itself, adds them in
+// a fixed order: loss and gradient repeat bit for bit.
 constexpr uint32_t REDUCE_SPLIT = 8;
-template <bool ADAM>
-__global__ void __launch_bounds__(32 * REDUCE_SPLIT) k_guide_reduce(GuideTrainArgs a, uint32_t n, float* p, float* m,
-                                                                    float* v, uint8_t* wpack, GuideAdam h) {
+__global__ void k_guide_reduce(const float* __restrict__ partial, GuideTrainArgs a, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (uint32_t)GUIDE_PARAMS) return;
+    float s0 = 0.0f, s1 = 0.0f;
+    uint32_t b = blockIdx.y;
+    for (; b + REDUCE_SPLIT < n; b += 2 * REDUCE_SPLIT) {
+        s0 += partial[(size_t)b * GUIDE_PARAMS + i];
+        s1 += partial[(size_t)(b + REDUCE_SPLIT) * GUIDE_PARAMS + i];
+    }
+    if (b < n) s0 += partial[(size_t)b * GUIDE_PARAMS + i];
+    const float s = s0 + s1;
+    if (s != 0.0f) atomicAdd(&a.grad[i], s);
+    if (blockIdx.x == 0 && blockIdx.y == REDUCE_SPLIT - 1 && threadIdx.x < 32) add_losses(a, n, threadIdx.x);
+}
+
+__global__ void __launch_bounds__(32 * REDUCE_SPLIT) k_guide_reduce_ordered(GuideTrainArgs a, uint32_t n) {
     __shared__ float part[REDUCE_SPLIT][32];
     const uint32_t lane = threadIdx.x & 31u, y = threadIdx.x >> 5;
     const uint32_t i = blockIdx.x * 32 + lane;  // GUIDE_PARAMS is a multiple of 32
@@ -556,42 +595,31 @@ __global__ void __launch_bounds__(32 * REDUCE_SPLIT) k_guide_reduce(GuideTrainAr
     }
     if (b < n) s0 += a.partial[(size_t)b * GUIDE_PARAMS + i];
     part[y][lane] = s0 + s1;
-    if (blockIdx.x == 0 && y == 1) {  // the batch's loss, one warp
-        double l = 0.0, c = 0.0;
-        for (uint32_t k = lane; k < n; k += 32) {
-            l += a.loss[k].x;
-            c += a.loss[k].y;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            l += __shfl_xor_sync(0xffffffffu, l, o);
-            c += __shfl_xor_sync(0xffffffffu, c, o);
-        }
-        if (lane == 0) {
-            a.stats[0] += (float)l;
-            a.stats[1] += (float)c;
-        }
-    }
+    if (blockIdx.x == 0 && y == 1) add_losses(a, n, lane);
     __syncthreads();
     if (y != 0) return;
     float gi = a.grad[i];
 #pragma unroll
     for (uint32_t k = 0; k < REDUCE_SPLIT; ++k) gi += part[k][lane];
-    if constexpr (ADAM) {
-        const float t = (float)max(*a.step, 1u);
-        const float mi = h.beta1 * m[i] + (1.0f - h.beta1) * gi;
-        const float vi = h.beta2 * v[i] + (1.0f - h.beta2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float mhat = mi / (1.0f - powf(h.beta1, t));
-        const float vhat = vi / (1.0f - powf(h.beta2, t));
-        const float pi = p[i] - h.lr * mhat / (sqrtf(vhat) + h.eps);
-        p[i] = pi;
-        pack_param(wpack, i, pi);
-        a.grad[i] = 0.0f;
-    } else {
-        a.grad[i] = gi;
-    }
+    a.grad[i] = gi;
+}
+
+// Adam on the FP32 master weights; clears the gradient and rewrites the weights' BF16 image.
+__global__ void k_guide_adam(GuideAdamState st, float* g, const uint32_t* step) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= GUIDE_PARAMS) return;
+    const float gi = g[i];
+    g[i] = 0.0f;
+    const float t = (float)max(*step, 1u);
+    const float mi = st.h.beta1 * st.m[i] + (1.0f - st.h.beta1) * gi;
+    const float vi = st.h.beta2 * st.v[i] + (1.0f - st.h.beta2) * gi * gi;
+    st.m[i] = mi;
+    st.v[i] = vi;
+    const float mhat = mi / (1.0f - powf(st.h.beta1, t));
+    const float vhat = vi / (1.0f - powf(st.h.beta2, t));
+    const float pi = st.p[i] - st.h.lr * mhat / (sqrtf(vhat) + st.h.eps);
+    st.p[i] = pi;
+    pack_param(st.wpack, i, pi);
 }
 
 __global__ void k_guide_pack(const float* p, uint8_t* wpack) {
@@ -721,11 +749,13 @@ void launch_guide_train(const GuideTrainArgs& a, const GuideAdamState* adam, cud
     uint32_t grid = (a.n + 127) / 128;
     if (grid == 0) return;
     k_guide_train<<<grid, 256, TRAIN_SMEM, s>>>(a);
-    static_assert(GUIDE_PARAMS % 32 == 0, "k_guide_reduce takes whole warps of parameters");
-    if (adam)
-        k_guide_reduce<true><<<GUIDE_PARAMS / 32, 32 * REDUCE_SPLIT, 0, s>>>(a, grid, adam->p, adam->m, adam->v, adam->wpack, adam->h);
-    else
-        k_guide_reduce<false><<<GUIDE_PARAMS / 32, 32 * REDUCE_SPLIT, 0, s>>>(a, grid, nullptr, nullptr, nullptr, nullptr, GuideAdam{});
+    if (adam) {
+        k_guide_reduce<<<dim3((GUIDE_PARAMS + 255) / 256, REDUCE_SPLIT), 256, 0, s>>>(a.partial, a, grid);
+        k_guide_adam<<<(GUIDE_PARAMS + 255) / 256, 256, 0, s>>>(*adam, a.grad, a.step);
+    } else {
+        static_assert(GUIDE_PARAMS % 32 == 0, "k_guide_reduce_ordered takes whole warps of parameters");
+        k_guide_reduce_ordered<<<GUIDE_PARAMS / 32, 32 * REDUCE_SPLIT, 0, s>>>(a, grid);
+    }
 }
 
 void launch_guide_pack(const float* p, uint8_t* wpack, cudaStream_t s) {

@@ -694,7 +694,7 @@ bg_status bg_render_guided(bg_ctx* ctx, const bg_scene* s, bg_guide* g, const bg
         float train_ms = 0.0f;
         if (record && pool_n >= 128) {
             int nb = train_batches(g, g->pool, pool_n, g->o.epochs, &g->epochs_done);
-            launches += g->o.epochs + 2 * (uint64_t)nb;
+            launches += g->o.epochs + 3 * (uint64_t)nb;
             CK(cudaGetLastError());
             CK(cudaEventRecord(g->ev[2], ctx->stream));
             float ls[2] = {0, 0};

@@ -58,8 +58,8 @@ constexpr int GUIDE_MAX_RANGES = 3;
 void launch_guide_infer(const uint8_t* wpack, const float4* query, const uint32_t* counts, uint32_t nranges,
                         uint32_t stride, float* out, bool mixture, uint32_t* err, int sms, cudaStream_t s);
 // Forward + backward of a.n samples (one CTA per 128) and the reduction of their partial
-// gradients into a.grad; with `adam`, an Adam step on the accumulated gradient, which is cleared
-// (two launches).
+// gradients into a.grad: for the gradient alone (`adam` null, two launches) in a fixed order, with
+// `adam` as they arrive, followed by an Adam step on the accumulated gradient, which is cleared (three).
 void launch_guide_train(const GuideTrainArgs& a, const GuideAdamState* adam, cudaStream_t s);
 void launch_guide_pack(const float* p, uint8_t* wpack, cudaStream_t s);
 // wsum[2b], wsum[2b + 1] = sums of the positive finite indirect (head 0) and direct (head 1)
