@@ -1637,7 +1637,7 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
     if (n > 65536) return fail(ctx, BG_ERR_INVALID, "at most 65536 scenes per batch");
     uint64_t total_pix = 0, total_items = 0;
     uint32_t max_depth = 0;
-    uint32_t variants = 0;  // bit 0: some scene is textured, bit 1: some scene holds an infinite light, 2-5: material classes
+    uint32_t variants = 0;  // as launch_wave_batch
     for (size_t i = 0; i < n; ++i) {
         const bg_batch_item& it = items[i];
         bg_render_opts o = it.opts;
@@ -1709,6 +1709,11 @@ bg_status bg_render_batch(bg_ctx* ctx, const bg_batch_item* items, size_t n, bg_
     if ((st = ensure_wave_for(ctx, total_items, &cap)) != BG_OK) {
         dfree_all(ctx, tmp);
         return st;
+    }
+    for (size_t i = 0; i < n; ++i) {
+        const uint64_t npix = (uint64_t)items[i].camera.width * items[i].camera.height;
+        if (items[i].opts.spp >= bg::FILM_SPLIT && bg::film_parts(npix, std::min<uint64_t>(cap, npix * items[i].opts.spp)) > 1)
+            variants |= 64u;
     }
     CK(cudaMemsetAsync(ctx->wave.ray_stats, 0, 4 * sizeof(unsigned long long), ctx->stream));
     // every wave of the batch in one CUDA graph, captured once per batch shape and replayed: the

@@ -386,12 +386,33 @@ __global__ void __launch_bounds__(128) k_emit_pending(Scene sc, WaveBuffers wb, 
     }
 }
 
+// The slots of a wave that hold thread slot i's film: [first, end), npix pixels in turn; `parts` threads share
+// a pixel (film_parts).
+struct FilmSpan {
+    uint64_t first, end, npix;
+    uint32_t parts;
+};
+template <bool MULTI>
+BG_D FilmSpan film_span(const RenderParams& rp, const SceneRender* sr, uint64_t item0, uint32_t n) {
+    FilmSpan f{0, n, (uint64_t)rp.width * rp.height, 1u};
+    if (MULTI) {
+        const uint64_t s0 = sr->item0, s1 = s0 + f.npix * rp.spp;
+        f.first = s0 > item0 ? s0 - item0 : 0;
+        f.end = min((uint64_t)n, s1 - item0);
+    }
+    if (rp.spp >= FILM_SPLIT) f.parts = film_parts(f.npix, f.end - f.first);
+    return f;
+}
+
 // Adds a wave's paths (items item0 .. item0 + n - 1 in slots 0 .. n - 1) to the film: their radiance
 // in L plus the last vertex's light contribution where its shadow rays have just resolved it, after
 // the radiance sanity checks of SamplerIntegrator::render (src/base/integrator.rs:91-120;
 // FilmTile::add_sample with the box filter, weight 1 to the sample's own pixel).  One thread adds all
 // of the wave's samples of a pixel, in sample order and without atomics (six FP64 atomics and one
-// integer one per path before: the Cornell box's contended 2^20 samples 0.12 ms of 1.86).
+// integer one per path before: the Cornell box's contended 2^20 samples 0.12 ms of 1.86).  Where that
+// leaves few threads with many samples each, `parts` threads share a pixel (film_parts): thread
+// slot i takes samples i, i + width, ... (width = npix * parts), and k_film_parts adds their sums, which stay
+// in slots of the ended paths' ray and throughput arrays until then.
 // CTL: the wave is wb.wavectl's of `total` items.  MULTI: pixels and films of the path's scene.
 template <bool MULTI, bool CTL>
 __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmBuffers film0, WaveBuffers wb,
@@ -403,15 +424,9 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
     }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const SceneRender* sr = MULTI ? tab + wb.scene_id[i] : nullptr;
-        const RenderParams& rp = pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr);
-        const uint64_t npix = (uint64_t)rp.width * rp.height;
-        uint64_t first = 0, end = n;  // the scene's slots in this wave
-        if (MULTI) {
-            const uint64_t s0 = sr->item0, s1 = s0 + npix * rp.spp;
-            first = s0 > item0 ? s0 - item0 : 0;
-            end = min((uint64_t)n, s1 - item0);
-        }
-        if (i - first >= npix) {  // a later sample of its pixel
+        const FilmSpan span = film_span<MULTI>(pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr), sr, item0, n);
+        const uint64_t width = span.npix * span.parts;
+        if (i - span.first >= width) {  // a later sample of its pixel
             if (MULTI) continue;
             break;
         }
@@ -421,21 +436,21 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
         float ps[3] = {0.0f, 0.0f, 0.0f};
         uint32_t cnt = 0, nan = 0;
         // four samples' loads in flight
-        for (uint64_t j0 = i; j0 < end; j0 += 4 * npix) {
+        for (uint64_t j0 = i; j0 < span.end; j0 += 4 * width) {
             float4 l4[4];
             uint32_t st[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const uint64_t j = j0 + k * npix;
-                if (j < end) {
+                const uint64_t j = j0 + k * width;
+                if (j < span.end) {
                     l4[k] = wb.L[j];
                     st[k] = wb.state[j];
                 }
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const uint64_t j = j0 + k * npix;
-                if (j >= end) break;
+                const uint64_t j = j0 + k * width;
+                if (j >= span.end) break;
                 RGB L = apply_pending(wb, (uint32_t)j, rgb(l4[k].x, l4[k].y, l4[k].z), st[k], nlights);
                 const float y = luminance(L);
                 if (is_nan(L) || y < -1e-5f || isinf(y)) {
@@ -455,6 +470,19 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
                 ++cnt;
             }
         }
+        if (nan) atomicAdd(f.nan_count, (unsigned long long)nan);
+        if (span.parts > 1) {
+            reinterpret_cast<double2*>(wb.ray_o)[i] = make_double2(s[0], s[1]);
+            reinterpret_cast<double2*>(wb.ray_d)[i] = make_double2(s[2], q[0]);
+            reinterpret_cast<double2*>(wb.beta)[i] = make_double2(q[1], q[2]);
+            if (f.pass) {
+                float* o = reinterpret_cast<float*>(wb.cls_queue) + 3 * (size_t)i;  // 5 words per slot
+                o[0] = ps[0];
+                o[1] = ps[1];
+                o[2] = ps[2];
+            }
+            continue;
+        }
         const size_t pix = wb.pixel[i];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -463,8 +491,67 @@ __global__ void __launch_bounds__(256) k_film(Scene sc0, RenderParams rp0, FilmB
             if (f.pass) f.pass[3 * pix + c] += ps[c];
         }
         f.count[pix] += cnt;
-        if (nan) atomicAdd(f.nan_count, (unsigned long long)nan);
     }
+}
+
+// Adds the sums that the threads sharing a pixel have left behind, in their order.
+template <bool MULTI, bool CTL>
+__global__ void __launch_bounds__(256) k_film_parts(RenderParams rp0, FilmBuffers film0, WaveBuffers wb, uint64_t item0,
+                                                    uint32_t n, uint64_t total, const SceneRender* tab) {
+    if (CTL) {
+        const WaveItems w = wave_items(wb, total);
+        item0 = w.item0;
+        n = w.n;
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const SceneRender* sr = MULTI ? tab + wb.scene_id[i] : nullptr;
+        const FilmSpan span = film_span<MULTI>(pick<MULTI>(rp0, MULTI ? &sr->rp : nullptr), sr, item0, n);
+        if (span.parts == 1 || i - span.first >= span.npix) {
+            if (MULTI) continue;
+            break;
+        }
+        const FilmBuffers& f = pick<MULTI>(film0, MULTI ? &sr->film : nullptr);
+        double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        float ps[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+        for (uint32_t p = 0; p < span.parts; ++p) {
+            const size_t j = i + p * span.npix;
+            const double2 a = reinterpret_cast<const double2*>(wb.ray_o)[j], b = reinterpret_cast<const double2*>(wb.ray_d)[j],
+                          c = reinterpret_cast<const double2*>(wb.beta)[j];
+            s[0] += a.x;
+            s[1] += a.y;
+            s[2] += b.x;
+            s[3] += b.y;
+            s[4] += c.x;
+            s[5] += c.y;
+            if (f.pass) {
+                const float* o = reinterpret_cast<const float*>(wb.cls_queue) + 3 * j;
+                ps[0] += o[0];
+                ps[1] += o[1];
+                ps[2] += o[2];
+            }
+        }
+        const size_t pix = wb.pixel[i];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            f.sum[3 * pix + c] += s[c];
+            f.sumsq[3 * pix + c] += s[3 + c];
+            if (f.pass) f.pass[3 * pix + c] += ps[c];
+        }
+        f.count[pix] += (uint32_t)((span.end - i + span.npix - 1) / span.npix);
+    }
+}
+
+// A wave's film launches (n = the paths of a full wave); returns their number.  split: some scene's
+// pixels may be shared by several threads.
+template <bool MULTI, bool CTL>
+static int launch_film(const Scene& sc, const RenderParams& rp, const FilmBuffers& film, const WaveBuffers& wb,
+                       uint64_t item0, uint32_t n, uint64_t total, const SceneRender* tab, bool split,
+                       const LaunchShape& ls, cudaStream_t s) {
+    k_film<MULTI, CTL><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, item0, n, total, tab);
+    if (!split) return 1;
+    k_film_parts<MULTI, CTL><<<ls.sms * 8, 256, 0, s>>>(rp, film, wb, item0, n, total, tab);
+    return 2;
 }
 
 static int launch_bounces(const Scene& sc, const RenderParams& rp, const WaveBuffers& wb, uint32_t* err,
@@ -516,13 +603,13 @@ int launch_wave(const Scene& sc, const Camera& cam, const RenderParams& rp, cons
                 cudaStream_t s, cudaEvent_t* ev, const GuideWave* gw) {
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_generate<<<grid, block, 0, s>>>(cam, rp, wb, item0, nitems);
-    int launches = 2 + launch_bounces(sc, rp, wb, err, ls, s, ev, gw);
+    int launches = 1 + launch_bounces(sc, rp, wb, err, ls, s, ev, gw);
     if (gw && (gw->flags & GW_RECORD)) {
         k_emit_pending<<<grid, block, 0, s>>>(sc, wb, *gw, nitems);
         launches += 1;
     }
-    k_film<false, false><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, item0, nitems, 0, nullptr);
-    return launches;
+    const bool split = rp.spp >= FILM_SPLIT && film_parts((uint64_t)rp.width * rp.height, nitems) > 1;
+    return launches + launch_film<false, false>(sc, rp, film, wb, item0, nitems, 0, nullptr, split, ls, s);
 }
 
 int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_depth, const WaveBuffers& wb,
@@ -534,26 +621,27 @@ int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_dep
     const FilmBuffers film{};
     const dim3 bin_grid(ls.sms * 4);
     k_generate_batch<<<grid, block, 0, s>>>(tab, nscenes, wb, item0, nitems);
-    int launches = 2;
+    int launches = 1;
     for (uint32_t b = 0; b <= max_depth; ++b) {
         k_extend<8, true><<<grid, block, 0, s>>>(sc, wb, b, err, ls.refill, tab, false);
         k_bin<true><<<bin_grid, BIN_BLOCK, 0, s>>>(sc, wb, b, tab);
-        launches += 2 + launch_shade_batch(tab, wb, b, err, variants >> 2, 2 * (uint32_t)ls.sms, ls.fork, s, (variants & 3u) != 0);
+        launches += 2 + launch_shade_batch(tab, wb, b, err, (variants >> 2) & 15u, 2 * (uint32_t)ls.sms, ls.fork, s, (variants & 3u) != 0);
         if (b < max_depth) {
             k_shadow<8, true><<<grid, block, 0, s>>>(sc, wb, err, ls.refill, tab);
             launches += 1;
         }
     }
-    k_film<true, false><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, item0, nitems, 0, tab);
-    return launches;
+    return launches + launch_film<true, false>(sc, rp, film, wb, item0, nitems, 0, tab, (variants & 64u) != 0, ls, s);
 }
 
 int launch_wave_chain(const Scene& sc, const Camera& cam, const RenderParams& rp, const FilmBuffers& film,
                       const WaveBuffers& wb, uint64_t total, uint32_t* err, const LaunchShape& ls, cudaStream_t s) {
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_generate_ctl<<<grid, block, 0, s>>>(cam, rp, wb, total);
-    int n = 3 + launch_bounces(sc, rp, wb, err, ls, s, nullptr, nullptr);
-    k_film<false, true><<<ls.sms * 8, 256, 0, s>>>(sc, rp, film, wb, 0, 0, total, nullptr);
+    int n = 2 + launch_bounces(sc, rp, wb, err, ls, s, nullptr, nullptr);
+    const uint64_t full = std::min<uint64_t>(total, wb.capacity);
+    const bool split = rp.spp >= FILM_SPLIT && film_parts((uint64_t)rp.width * rp.height, full) > 1;
+    n += launch_film<false, true>(sc, rp, film, wb, 0, 0, total, nullptr, split, ls, s);
     k_wave_advance<<<1, 32, 0, s>>>(wb);
     return n;
 }

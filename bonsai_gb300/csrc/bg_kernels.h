@@ -196,6 +196,24 @@ void launch_tree_integrator(int kind, bool ref_compat, int layout, const Scene& 
                             cudaStream_t s);
 void launch_megakernel(bool ref_compat, const Scene& sc, const Camera& cam, const RenderParams& rp,
                        const FilmBuffers& film, uint32_t* err, const LaunchShape& ls, cudaStream_t s);
+// Threads that share a pixel in the film pass of a wave with `paths` paths over npix pixels: 1, unless a
+// pixel has FILM_SPLIT samples or more and the pixels alone are fewer threads than FILM_THREADS (nearly all
+// that are resident); then about the root of the samples, so that summing the samples and summing the
+// threads take equally long.
+// Cornell box, one thread a pixel / this / an atomic add per path: 1 x 1 pixels and 2^20 samples 702 / 3.1 / 8.8 ms,
+// 8 x 8 and 2^16 87.3 / 6.1 / 10.3, 16 x 16 and 2^14 27.1 / 5.9 / 8.5, 64 x 64 and 2^10 6.8 / 5.5 / 8.0; with
+// 256 x 256 pixels and 64 samples one thread a pixel costs nothing (5.5 / 5.5 / 7.9).
+constexpr uint32_t FILM_SPLIT = 256, FILM_THREADS = 1u << 18;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t film_parts(uint64_t npix, uint64_t paths) {
+    const uint64_t m = (paths + npix - 1) / npix;
+    if (m < FILM_SPLIT) return 1;
+    uint64_t p = 1;
+    while (4 * p * p <= m && 2 * p * npix <= FILM_THREADS) p *= 2;
+    return (uint32_t)p;
+}
 // One wave of the PBRT wavefront: items [item0, item0 + nitems) of the pixel x sample space.
 // Returns the number of kernels launched.  stage_events (optional): 4 events per bounce, recorded
 // before extend, before shade, before shadow and after it.
@@ -213,7 +231,8 @@ int launch_wave_chain(const Scene& sc, const Camera& cam, const RenderParams& rp
 // `nscenes` scenes (tab, device); paths of all scenes share the queues of one set of launches
 // (8-wide BVH layouts).  max_depth = the largest of the scenes'.  Returns the kernels launched.
 // variants: bit 0 some scene is textured, bit 1 some scene holds an infinite light (the shade
-// launches then take the variants that handle both per scene), bits 2-5 the scenes' material classes.
+// launches then take the variants that handle both per scene), bits 2-5 the scenes' material classes,
+// bit 6 some scene's pixels are shared by threads of the film pass (film_parts).
 int launch_wave_batch(const SceneRender* tab, uint32_t nscenes, uint32_t max_depth, const WaveBuffers& wb,
                       uint64_t item0, uint32_t nitems, uint32_t* err, const LaunchShape& ls, cudaStream_t s,
                       uint32_t variants = 0);
