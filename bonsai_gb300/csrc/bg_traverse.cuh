@@ -525,8 +525,11 @@ BG_D void octant_table_fill(uint8_t* perm) {
 // comes as 1024 + b (byte_plus_1024) and meets O - 1024 A, rounded down for the near planes and up
 // for the far planes: an error of at most A 2^-13 byte steps, so boxes only grow.  Two planes share
 // one packed multiply-add.  A box is missed when k * min(far planes, t_max) - max(near planes, 0)
-// is negative; the sign bits are collected by funnel shifts.  A NaN plane (0 * infinity in scenes of
-// more than 2^110 in extent) is ignored by min / max.
+// is negative; the sign bits are collected by funnel shifts.  O - 1024 A is one directed multiply-add: where
+// 1024 A alone exceeds FP32 (a zero direction component, |idir| = 1e20, and a node more than 2^59 in extent) its
+// bounds are the largest finite number on the one side and infinity on the other, and the box only
+// grows again.  That holds to an extent of 2^61.5, where (p - o) * idir itself ends; beyond, an axis with a zero
+// component no longer decides for the right box.  A NaN plane (A infinite) is ignored by min / max.
 // The loop is bound by instruction issue, the half-rate ALU pipe first: a half-to-float conversion
 // runs beside it, an integer one or a byte permute per plane does not.  Closest and any hit of
 // 16.8M rays over 2.1M triangles: 13.75 ms with shift / mask / convert and scalar multiply-adds,
@@ -543,11 +546,10 @@ BG_D void bvh8_node_hits(const Scene& sc, uint32_t ni, const Ray8& r, float t_ma
     const uint32_t imask = ebits >> 24;
     const V3 aidir = v3(sx * r.idir.x, sy * r.idir.y, sz * r.idir.z);
     const V3 aorig = v3((n0.x - r.o.x) * r.idir.x, (n0.y - r.o.y) * r.idir.y, (n0.z - r.o.z) * r.idir.z);
-    const V3 shift = 1024.0f * aidir;  // exact
     const float2 axy = make_float2(aidir.x, aidir.y), azz = make_float2(aidir.z, aidir.z);
-    const float2 near_xy = make_float2(__fsub_rd(aorig.x, shift.x), __fsub_rd(aorig.y, shift.y));
-    const float2 far_xy = make_float2(__fsub_ru(aorig.x, shift.x), __fsub_ru(aorig.y, shift.y));
-    const float2 near_far_z = make_float2(__fsub_rd(aorig.z, shift.z), __fsub_ru(aorig.z, shift.z));
+    const float2 near_xy = make_float2(__fmaf_rd(-1024.0f, aidir.x, aorig.x), __fmaf_rd(-1024.0f, aidir.y, aorig.y));
+    const float2 far_xy = make_float2(__fmaf_ru(-1024.0f, aidir.x, aorig.x), __fmaf_ru(-1024.0f, aidir.y, aorig.y));
+    const float2 near_far_z = make_float2(__fmaf_rd(-1024.0f, aidir.z, aorig.z), __fmaf_ru(-1024.0f, aidir.z, aorig.z));
     const uint32_t qlx[2] = {__float_as_uint(n2.x), __float_as_uint(n2.y)};
     const uint32_t qly[2] = {__float_as_uint(n2.z), __float_as_uint(n2.w)};
     const uint32_t qlz[2] = {__float_as_uint(n3.x), __float_as_uint(n3.y)};
