@@ -3,7 +3,7 @@
 Tunes, by coordinate descent on short renders of the actual scene (device-timed with the
 library's CUDA events, L2 flushed before each trial):
   refill        - traversal: lanes a warp lets go idle before it fetches new rays (32 = whole warp)
-  blocks_per_sm - persistent grid of the wavefront stages
+  blocks_per_sm - persistent grid of generation and traversal
   wave_paths    - paths per wave (queue capacity)
   sort_rays     - bin each bounce's extension rays by direction octant and origin cell
   concurrent_shade - run a bounce's material-class shade kernels side by side

@@ -15,8 +15,6 @@
 // so both produce the same estimate for every sample up to float summation order.  The direct
 // strategy of MIS through the BSDF becomes an occlusion ray up to the light (the light's own
 // triangle skipped), as in the path wavefront.
-#include <algorithm>
-
 #include "bg_tree_wave.cuh"
 
 #ifndef BG_MINBLOCKS
@@ -143,7 +141,7 @@ int launch_tree_wave(int kind, const Scene& sc, const Camera& cam, const RenderP
     dim3 grid(ls.sms * ls.blocks_per_sm), block(128);
     k_tw_gen<<<grid, block, 0, s>>>(cam, rp, tw, item0, n);
     ++launches;
-    const dim3 shade_grid(std::max(1u, (uint32_t)(ls.sms * ls.blocks_per_sm) * 128u / TW_SHADE_BLOCK));
+    const dim3 shade_grid(ls.sms);  // one block of TW_SHADE_BLOCK fits an SM
     const bool wide8 = sc.nodes8 != nullptr;
     for (uint32_t d = 0; d < rp.max_depth; ++d) {
         if (wide8) launch_chained(k_tw_extend<8>, grid, block, s, sc, tw, d, err, ls.refill);
