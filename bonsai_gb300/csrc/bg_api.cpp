@@ -302,7 +302,7 @@ bg_status ensure_wave(bg_ctx* ctx, uint32_t cap) {
 }
 
 uint32_t wave_limit(const bg_ctx* ctx) {
-    if (ctx->max_queue != kDefaultQueue) return ctx->max_queue;
+    if (ctx->max_queue) return ctx->max_queue;
     return ctx->cap ? kFallbackQueue : ctx->queue_fit;
 }
 
@@ -310,7 +310,7 @@ bg_status ensure_wave_for(bg_ctx* ctx, uint64_t total, uint32_t* cap) {
     for (;;) {
         *cap = (uint32_t)std::min<uint64_t>(wave_limit(ctx), std::max<uint64_t>(total, 1));
         const bg_status st = ensure_wave(ctx, *cap);
-        if (st != BG_ERR_OOM || ctx->max_queue != kDefaultQueue || *cap <= kFallbackQueue) return st;
+        if (st != BG_ERR_OOM || ctx->max_queue || *cap <= kFallbackQueue) return st;
         cudaGetLastError();  // the failed allocation's
         ctx->queue_fit = std::max(kFallbackQueue, *cap / 2);
     }
@@ -521,7 +521,7 @@ bg_status bg_create(const bg_device_opts* opts, bg_ctx** out) {
     }
     if (opts) {
         ctx->cap = opts->memory_cap_bytes;
-        if (opts->max_queue_paths) ctx->max_queue = opts->max_queue_paths;
+        ctx->max_queue = opts->max_queue_paths;
         if (opts->block_size) ctx->shape.block = (int)opts->block_size;
     }
     auto bail = [&](cudaError_t e) {
@@ -639,7 +639,7 @@ bg_status bg_memcpy_d2h(bg_ctx* ctx, void* h, const void* d, size_t bytes) {
 
 bg_status bg_get_tuning(const bg_ctx* ctx, bg_tuning* out) {
     if (!ctx || !out) return BG_ERR_INVALID;
-    out->wave_paths = ctx->max_queue;
+    out->wave_paths = wave_limit(ctx);
     out->blocks_per_sm = (uint32_t)ctx->shape.blocks_per_sm;
     out->refill = (uint32_t)ctx->shape.refill;
     out->flags = (ctx->shape.sort_rays ? BG_TUNE_SORT_RAYS : 0u) | (ctx->shape.l2_persist ? BG_TUNE_L2_PERSIST : 0u) |
@@ -1544,7 +1544,7 @@ bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const 
                 const uint64_t nl = std::max<uint64_t>(s->dev.nlights, 1);
                 const uint64_t per_node = kind == 1 ? nl : (kind == 2 ? 2 * nl : 2);
                 const uint64_t sh_budget = 1ull << 25;  // shadow rays per level
-                uint64_t W = std::min<uint64_t>({(uint64_t)kTreeWaveSamples, (uint64_t)ctx->max_queue, total,
+                uint64_t W = std::min<uint64_t>({(uint64_t)kTreeWaveSamples, (uint64_t)wave_limit(ctx), total,
                                                  std::max<uint64_t>(1, sh_budget / (2 * per_node))});
                 W = std::max<uint64_t>(W, 1);
                 const bool textured = s->dev.ntex > 0;

@@ -25,7 +25,7 @@ struct bg_ctx {
     uint64_t cap = 0, used = 0;
     bg::ShadeFork fork{};           // streams / events of BG_TUNE_CONCURRENT_SHADE
     bg::LaunchShape shape{1, 128};
-    uint32_t max_queue = kDefaultQueue;
+    uint32_t max_queue = 0;              // paths per wave set by the caller (0: the library's choice)
     uint32_t queue_fit = kDefaultQueue;  // the largest default wave that has not failed to allocate
     uint32_t* d_err = nullptr;
     // what a call reads back about its launches, page-locked so that the copies queue up behind the
@@ -119,8 +119,8 @@ void dfree_all(bg_ctx* ctx, std::vector<void*>& v);
 bg::Camera make_camera(const bg_camera& c);
 bg_status ensure_film(bg_ctx* ctx, uint32_t w, uint32_t h);
 bg_status ensure_wave(bg_ctx* ctx, uint32_t cap);
-// Paths per wave before a render's own total bounds them; ensure_wave for `total` paths (*cap = paths
-// per wave).
+// Paths per wave before a render's own total bounds them (a size set by the caller as it is, else the
+// library's choice); ensure_wave for `total` paths (*cap = paths per wave).
 uint32_t wave_limit(const bg_ctx* ctx);
 bg_status ensure_wave_for(bg_ctx* ctx, uint64_t total, uint32_t* cap);
 bg_status check_device_error(bg_ctx* ctx, uint32_t* word);

@@ -315,7 +315,9 @@ bg_status bg_scene_commit(bg_scene* scene, uint32_t bvh_kind, bg_build_stats* st
 
 /* ---- launch tuning (chosen by the autotuner in bonsai_gb300/autotune.py) --------------------- */
 typedef struct bg_tuning {
-    uint32_t wave_paths;    /* wavefront capacity: paths per wave                                  */
+    uint32_t wave_paths;    /* wavefront capacity: paths per wave.  Once set it is taken as it is (240
+                               bytes of device memory a path, or BG_ERR_OOM); until then the
+                               library chooses, and bg_get_tuning says what it would take now     */
     uint32_t blocks_per_sm; /* persistent grid of generation and traversal = SMs x blocks_per_sm
                                (blocks of 128 threads; shading and binning fill the SMs by themselves) */
     uint32_t refill;        /* traversal: a warp fetches new rays once this many lanes are idle
