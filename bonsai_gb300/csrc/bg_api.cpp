@@ -35,7 +35,14 @@ bg_status dalloc(bg_ctx* ctx, size_t bytes, void** p, std::vector<void*>* owner)
         return fail(ctx, BG_ERR_OOM, "device memory cap exceeded (" + std::to_string(ctx->used + bytes) + " > " +
                                          std::to_string(ctx->cap) + " bytes)");
     cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
+    if (e == cudaErrorMemoryAllocation && release_wave(ctx)) {
+        cudaGetLastError();  // the failed allocation's
+        e = cudaMalloc(p, bytes ? bytes : 16);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return cuda_fail(ctx, e, "cudaMalloc");
+    }
     ctx->used += bytes;
     ctx->sizes[*p] = bytes;
     if (owner) owner->push_back(*p);
@@ -301,17 +308,37 @@ bg_status ensure_wave(bg_ctx* ctx, uint32_t cap) {
     return BG_OK;
 }
 
+// Nothing allocates through `ctx` between ensure_wave and the end of a render's waves.
+bool release_wave(bg_ctx* ctx) {
+    if (ctx->wave.capacity <= std::max(kFallbackQueue, ctx->max_queue)) return false;
+    cudaStreamSynchronize(ctx->stream);
+    dfree_all(ctx, ctx->wave_allocs);
+    ctx->wave = bg::WaveBuffers{};
+    return true;
+}
+
 uint32_t wave_limit(const bg_ctx* ctx) {
     if (ctx->max_queue) return ctx->max_queue;
-    return ctx->cap ? kFallbackQueue : ctx->queue_fit;
+    if (ctx->cap) return kFallbackQueue;
+    uint32_t limit = ctx->queue_fit;
+    if (limit <= std::max(kFallbackQueue, ctx->wave.capacity)) return limit;  // already there
+    size_t free = 0, total = 0;
+    if (cudaSetDevice(ctx->device) != cudaSuccess || cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return kFallbackQueue;
+    }
+    const uint64_t avail = free + kWaveBytes * ctx->wave.capacity;  // a larger wave replaces the present one
+    while (limit > kFallbackQueue && kWaveBytes * limit > avail / kWaveShare) limit /= 2;
+    return std::max(limit, std::max(kFallbackQueue, ctx->wave.capacity));
 }
 
 bg_status ensure_wave_for(bg_ctx* ctx, uint64_t total, uint32_t* cap) {
     for (;;) {
-        *cap = (uint32_t)std::min<uint64_t>(wave_limit(ctx), std::max<uint64_t>(total, 1));
+        // the present wave and kFallbackQueue need no look at the free memory
+        const uint32_t have = ctx->max_queue || ctx->cap ? 0u : std::max(ctx->wave.capacity, kFallbackQueue);
+        *cap = (uint32_t)std::min<uint64_t>(total <= have ? have : wave_limit(ctx), std::max<uint64_t>(total, 1));
         const bg_status st = ensure_wave(ctx, *cap);
         if (st != BG_ERR_OOM || ctx->max_queue || *cap <= kFallbackQueue) return st;
-        cudaGetLastError();  // the failed allocation's
         ctx->queue_fit = std::max(kFallbackQueue, *cap / 2);
     }
 }
@@ -1544,7 +1571,7 @@ bg_status bg_render(bg_ctx* ctx, const bg_scene* s, const bg_camera* cam, const 
                 const uint64_t nl = std::max<uint64_t>(s->dev.nlights, 1);
                 const uint64_t per_node = kind == 1 ? nl : (kind == 2 ? 2 * nl : 2);
                 const uint64_t sh_budget = 1ull << 25;  // shadow rays per level
-                uint64_t W = std::min<uint64_t>({(uint64_t)kTreeWaveSamples, (uint64_t)wave_limit(ctx), total,
+                uint64_t W = std::min<uint64_t>({(uint64_t)kTreeWaveSamples, (uint64_t)(ctx->max_queue ? ctx->max_queue : kTreeWaveSamples), total,
                                                  std::max<uint64_t>(1, sh_budget / (2 * per_node))});
                 W = std::max<uint64_t>(W, 1);
                 const bool textured = s->dev.ntex > 0;

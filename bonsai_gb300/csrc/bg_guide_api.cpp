@@ -614,11 +614,11 @@ bg_status bg_render_guided(bg_ctx* ctx, const bg_scene* s, bg_guide* g, const bg
     const uint32_t pass_spp = (uint32_t)std::max<uint64_t>(1, g->o.pass_paths / npix);
     // a guided path holds 2 KB of records, queries and mixtures besides: waves of kFallbackQueue unless
     // the caller has chosen a size
-    const uint32_t queue = ctx->max_queue ? ctx->max_queue : std::min(kFallbackQueue, wave_limit(ctx));
+    const uint32_t queue = ctx->max_queue ? ctx->max_queue : kFallbackQueue;
     const uint32_t cap = (uint32_t)std::min<uint64_t>(queue, npix * std::min(pass_spp, std::max(o->spp, 1u)));
-    if ((st = ensure_wave(ctx, cap)) != BG_OK) return st;
     if ((st = ensure_guide_wave(g, cap)) != BG_OK) return st;
     if ((st = ensure_pass(g, npix)) != BG_OK) return st;
+    if ((st = ensure_wave(ctx, cap)) != BG_OK) return st;  // last: no allocation while it is in use
     bg::FilmBuffers film = ctx->film;
     film.pass = g->pass;
     const bg::Camera dc = make_camera(*cam);

@@ -13,10 +13,14 @@
 
 // Paths per wave unless the caller says otherwise.  Every stage of a wave ends with a few long rays on an
 // almost idle GPU (0.2 ms a bounce on the production scene), so fewer waves are better until the
-// path state (about 230 bytes a path, 7.7 GB here) is a burden: production frame at 16 spp (33M paths)
+// path state (240 bytes a path, 8.1 GB here) is a burden: production frame at 16 spp (33M paths)
 // 93.2 ms with waves of 2^22, 85.1 / 81.0 / 79.0 with 2^23 / 2^24 / 2^25; example scene (16.8M paths) 4.85 /
-// 4.33 / 4.08 / 4.08.  Under a memory cap, and where that much is not to be had, waves of kFallbackQueue.
+// 4.33 / 4.08 / 4.08.  Under a memory cap, and where that much is not to be had, waves of kFallbackQueue
+// (1.0 GB).  A context keeps its wave, so it takes no more than 1 / kWaveShare of the free memory for one
+// larger than kFallbackQueue (8.1 GB from 129 GB free on: a second context or another library finds the
+// rest), and gives such a wave back when another allocation of its own fails (release_wave).
 constexpr uint32_t kDefaultQueue = 1u << 25, kFallbackQueue = 1u << 22;
+constexpr uint64_t kWaveBytes = 240, kWaveShare = 16;  // bytes per path, as ensure_wave allocates
 
 struct bg_ctx {
     int device = 0;
@@ -119,6 +123,8 @@ void dfree_all(bg_ctx* ctx, std::vector<void*>& v);
 bg::Camera make_camera(const bg_camera& c);
 bg_status ensure_film(bg_ctx* ctx, uint32_t w, uint32_t h);
 bg_status ensure_wave(bg_ctx* ctx, uint32_t cap);
+// Frees a wave that the library chose larger than kFallbackQueue (not while one is in use).
+bool release_wave(bg_ctx* ctx);
 // Paths per wave before a render's own total bounds them (a size set by the caller as it is, else the
 // library's choice); ensure_wave for `total` paths (*cap = paths per wave).
 uint32_t wave_limit(const bg_ctx* ctx);

@@ -97,3 +97,64 @@ def test_setting_what_get_says_changes_nothing(gpu_ctx):
         assert np.array_equal(a.rgb, b.rgb) and a.stats.launches == b.stats.launches
     finally:
         ctx.close()
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+def _film(ctx, spp=32):
+    """A film of 2^20 pixels: 2^25 paths at 32 samples."""
+    sd = S.cornell(1024, 1024)
+    sc = G.Scene(ctx, sd, A.BG_BVH_WIDE)
+    try:
+        return G.PathIntegrator(sd.camera, spp, 3).render(sc).rgb
+    finally:
+        sc.close()
+
+
+def test_a_large_wave_makes_way_for_other_allocations():
+    """More than is free with the 8.1 GB wave, less than is free without it: the same context's next allocation
+    succeeds, and renders go on."""
+    ctx = G.Context(0)
+    try:
+        before = _free()
+        want = _film(ctx)
+        held = before - _free()
+        if held < 7 << 30:
+            pytest.skip("the device has too little free memory for the largest wave")
+        p = ctx.alloc(_free() + (4 << 30))
+        assert _free() > 1 << 30
+        ctx.free(p)
+        assert before - _free() < 1 << 30  # scene, film: the wave is gone
+        assert np.array_equal(_film(ctx), want)  # and comes back
+        assert before - _free() >= held - (1 << 28)
+    finally:
+        ctx.close()
+
+
+def test_a_wave_takes_a_share_of_the_free_memory():
+    """With 60 GB free a wave is at most 60 / 16 GB (2^23 paths, 2.0 GB), with 10 GB free 2^22 paths (1.0 GB), as
+    on a device with plenty the film is the same samples."""
+    other = G.Context(0)
+    plenty = G.Context(0)
+    try:
+        if _free() < 200 << 30:
+            pytest.skip("needs most of the device free")
+        want = _film(plenty)
+        plenty.close()
+        for leave, most in ((60 << 30, 60 << 26), (10 << 30, 240 << 22)):
+            p = other.alloc(_free() - leave)
+            ctx = G.Context(0)
+            try:
+                before = _free()
+                got = _film(ctx)
+                took = before - _free() - 64 * (1 << 20)  # less the film
+                assert took <= most + (64 << 20), (leave, took)
+                np.testing.assert_allclose(got, want, rtol=1e-6, atol=0)
+            finally:
+                ctx.close()
+                other.free(p)
+    finally:
+        other.close()
