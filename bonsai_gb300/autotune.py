@@ -9,12 +9,14 @@ library's CUDA events, L2 flushed before each trial):
   concurrent_shade - run a bounce's material-class shade kernels side by side
 and, by tune_layout, the traversal node width: the scene's BVH built 8-wide (BG_BVH_WIDE) and
 2-wide (BG_BVH_WIDE2), each timed on the same trial render.
-The result is cached as JSON keyed by GPU name, scene signature and render settings
-(default ~/.cache/bonsai_gb300/tuning.json, or $BONSAI_TUNING_CACHE).
+The result is cached as JSON keyed by GPU name, scene signature, render settings and the library's
+bytes (default ~/.cache/bonsai_gb300/tuning.json, or $BONSAI_TUNING_CACHE): a choice measured on other
+kernels is not applied to these.
 """
 from __future__ import annotations
 
 import ctypes as C
+import hashlib
 import json
 import os
 from pathlib import Path
@@ -42,9 +44,16 @@ def _gpu_name() -> str:
         return "unknown"
 
 
+def _library_id() -> str:
+    try:
+        return hashlib.sha1(A.LIB_PATH.read_bytes()).hexdigest()[:16]
+    except OSError:
+        return "none"
+
+
 def key_of(sd, spp: int) -> str:
     c = sd.camera
-    return f"{_gpu_name()}|tri{sd.ntri}|sph{sd.nsph}|{c.width}x{c.height}|depth{sd.max_depth}|spp{spp}|v4"
+    return f"{_gpu_name()}|tri{sd.ntri}|sph{sd.nsph}|{c.width}x{c.height}|depth{sd.max_depth}|spp{spp}|{_library_id()}"
 
 
 def get(ctx) -> A.bg_tuning:
@@ -85,7 +94,10 @@ def tune(ctx, scene, integrator, spp: int = 4, use_cache: bool = True, verbose: 
         c = cache[key]
         set_(ctx, c["refill"], c["blocks_per_sm"], c["wave_paths"], c.get("sort_rays", 0), c.get("concurrent_shade", 1))
         return dict(c, cached=True)
-    cur = {"refill": 32, "blocks_per_sm": 8, "wave_paths": 1 << 22, "sort_rays": 0, "concurrent_shade": 1}
+    t = get(ctx)  # the descent starts from the context's settings
+    cur = {"refill": t.refill, "blocks_per_sm": t.blocks_per_sm, "wave_paths": t.wave_paths,
+           "sort_rays": int(bool(t.flags & A.BG_TUNE_SORT_RAYS)),
+           "concurrent_shade": int(bool(t.flags & A.BG_TUNE_CONCURRENT_SHADE))}
     trials = []
 
     def run(cfg, tspp):
