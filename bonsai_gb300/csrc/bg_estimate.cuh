@@ -1,5 +1,5 @@
 // bg_estimate.cuh - per-thread ray queries over any BVH layout and estimate_direct for the
-// per-sample megakernels (the reference-layout path integrator, Whitted, direct lighting).
+// per-sample Whitted and direct-lighting kernels.
 #pragma once
 #include "bg_shading.cuh"
 #include "bg_traverse.cuh"
@@ -65,7 +65,5 @@ BG_D RGB estimate_direct_mk(const Scene& sc, const Isect& it, const BSDF& bsdf, 
     }
     return out;
 }
-
-// PathIntegrator::radiance (src/integrators/path.rs:51-146) over the reference BVH.
 
 }  // namespace bg

@@ -1,4 +1,4 @@
-// bg_film.cuh - film accumulation on the device (shared by the path wavefront, the megakernels and
+// bg_film.cuh - film accumulation on the device, one path at a time (the per-path kernel and
 // the Whitted / direct-lighting integrators).
 #pragma once
 #include "bg_kernels.h"

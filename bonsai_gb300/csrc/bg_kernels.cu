@@ -1,11 +1,11 @@
-// bg_kernels.cu - ray-query kernels, the per-path megakernel and the PBRT wavefront stages.
+// bg_kernels.cu - ray-query kernels and the PBRT wavefront stages.
 //
-// Wavefront (PBRT mode, 2-wide BVH):  one wave = up to `capacity` (pixel, sample) paths.
+// Wavefront (PBRT mode, 8-wide and 2-wide BVH):  one wave = up to `capacity` (pixel, sample) paths.
 //   generate -> [extend -> bin -> shade -> shadow] x (max_depth + 1) -> film
 // Queue sizes live in device memory; every stage launches a fixed persistent grid that reads its
 // own work count, so the chain needs no host synchronisation and can be captured in a CUDA graph.
-// Traversal stages pull 32-ray batches per warp from an atomic head (dynamic load balance);
-// queues are compacted with warp ballot + popc + one atomic per warp.
+// Traversal stages pull rays for a warp's idle lanes from an atomic head (dynamic load balance);
+// queues are compacted by whole blocks, one atomic per block and queue (BlockAppend).
 //
 // Renders over the reference layout (REF_COMPAT, and PBRT as a cross-check) run per path: bg_mega.cu.
 #include "bg_guide.cuh"
@@ -13,8 +13,6 @@
 #include "bg_kernels.h"
 #include "bg_shading.cuh"
 #include "bg_traverse.cuh"
-#include "bg_film.cuh"
-#include "bg_estimate.cuh"
 #include "bg_warp.cuh"
 #include "bg_wave.cuh"
 

@@ -873,8 +873,6 @@ BG_D RGB light_radiance_along(const Scene& sc, uint32_t light, V3 wi, V3 n_light
 // Whether a scene's light list holds more than triangles (the infinite light, emitting spheres or
 // quadrics): such scenes run the shade variants with the general light code.
 BG_HD bool general_lights(const Scene& sc) { return sc.inf || sc.sph_emis || sc.quad_emis; }
-// Light::radiance of every light for a ray that escapes the scene (only infinite lights emit).
-BG_D RGB escaped_radiance(const Scene& sc, V3 dir) { return sc.inf ? inf_radiance(sc, dir) : rgb(0.0f); }
 
 // ---- camera
 BG_D V3 xf_point(const float m[4][4], V3 p) {  // point3.rs:51-69

@@ -25,8 +25,8 @@ BG_D uint32_t warp_append(uint32_t* counter, bool pred) {
 }
 
 // Appends of a whole block to NQ queues with one atomic per queue: thread t enters counters[c]'s queue
-// when pred[c], at pos[c].  Every thread of the block calls it (two barriers); `sm` is the block's
-// scratch, free again after the next barrier.  Queue counters are single addresses, and a counter
+// when pred[c], at pos[c].  Every thread of the block calls it (two barriers); the struct is the block's
+// shared scratch, free again after the next barrier.  Queue counters are single addresses, and a counter
 // takes about one atomic per nanosecond from the whole GPU: one per warp and queue bound the binning
 // and most of the shading (2^20 Cornell box paths: binning 38 us a bounce, 3 us of memory traffic).
 template <int NQ>
@@ -66,7 +66,7 @@ struct BlockAppend {
 
 // A block's threads grouped by key (0 .. NK - 1): returns the thread whose item this thread takes, so
 // that warps hold one key each but for NK - 1 borders.  Every thread of the block calls it (three
-// barriers); `sm` is free again after the next barrier.
+// barriers); the struct is the block's shared scratch, free again after the next barrier.
 template <int NK>
 struct BlockGroup {
     uint32_t n[NK][32];

@@ -9,7 +9,6 @@
 #include "bg_kernels.h"
 #include "bg_shading.cuh"
 #include "bg_traverse.cuh"
-#include "bg_film.cuh"
 #include "bg_estimate.cuh"
 #include "bg_warp.cuh"
 
@@ -620,7 +619,7 @@ BG_D void shade_unit(const Scene& sc0, const RenderParams& rp0, const WaveBuffer
                   GWK && (gw.flags & GW_RECORD) != 0, err, out.lrec_emit, append);
 }
 
-// Shades a bounce's paths of material class CLS, one block per SM.
+// Shades a bounce's paths of material class CLS; one block fits an SM.
 template <int CLS, bool MULTI, bool GWK, bool TEX, bool INF, bool SHL>
 __global__ void __launch_bounds__(shade_block(GWK, TEX, INF), 1)
     k_shade(Scene sc0, RenderParams rp0, WaveBuffers wb, GuideWave gw, uint32_t bounce, uint32_t* err, const SceneRender* tab) {
