@@ -3,6 +3,8 @@
 Every sample must reach its pixel once.  The other arm renders the same samples in accumulated pieces of
 255 a pixel, where one thread adds a pixel's samples: the same paths, so FP64 sums of at most 70,000
 non-negative terms in another order, equal to 70,000 * 2^-53 = 8e-12 (1e-11 here)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -107,6 +109,23 @@ def test_guided_passes_keep_their_pass_film(gpu_ctx):
     finally:
         autotune.set_(gpu_ctx, old.refill, old.blocks_per_sm, old.wave_paths)
         sc.close()
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 70_001), (8, 8, 1025)])  # waves of 65,536 paths: two each
+def test_allocation_free_render(gpu_ctx, w, h, spp):
+    sd = S.cornell(w, h)
+    sc = G.Scene(gpu_ctx, sd, A.BG_BVH_WIDE)
+    want = G.PathIntegrator(sd.camera, spp, 4).render(sc).rgb
+    cam, o = G.camera_struct(sd.camera), A.bg_render_opts()
+    o.spp, o.max_depth, o.rr_threshold, o.mode = spp, 4, 1.0, A.BG_MODE_PBRT
+    d_out, got = gpu_ctx.alloc(w * h * 12), np.zeros((h, w, 3), np.float32)
+    try:
+        gpu_ctx.check(gpu_ctx.lib.bg_render_noalloc(sc.h, C.byref(cam), C.byref(o), d_out, None))
+        gpu_ctx.d2h(got, d_out)
+    finally:
+        gpu_ctx.free(d_out)
+        sc.close()
+    np.testing.assert_allclose(got, want, rtol=1e-6, atol=0)
 
 
 def test_few_pixels_take_no_longer_than_many(gpu_ctx):
